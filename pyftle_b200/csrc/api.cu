@@ -1,4 +1,5 @@
 // api.cu -- C ABI plumbing: error reporting, argument validation, packing dispatch.
+#include <math.h>
 #include <stdarg.h>
 #include <stdio.h>
 
@@ -54,6 +55,21 @@ int grid_from_abi(const ftle_grid *g, GridK *out) {
   if (nodes > (1LL << 40)) return fail_invalid("grid too large");
   out->periodic = g->periodic ? 1 : 0;
   out->nodes = nodes;
+  // The division by the reciprocal (grid_coords in plain_f64.cu) is exact for spacings well
+  // inside the exponent range and dividends that are not tiny; others are divided on scaled
+  // mantissas.
+  out->div_min = (1023u - 900u) << 20;
+  for (int a = 0; a < 3; ++a) {
+    const double s = out->spacing[a];
+    int e;
+    out->man[a] = 2.0 * frexp(s, &e);
+    out->man_exp[a] = e - 1;
+    if (!(e > -300 && e < 300)) out->div_min = 0x80000000u;
+    out->rcp_hi[a] = 1.0 / s;
+    out->rcp_lo[a] = fma(-out->rcp_hi[a], s, 1.0) / s;
+    out->man_hi[a] = 1.0 / out->man[a];
+    out->man_lo[a] = fma(-out->man_hi[a], out->man[a], 1.0) / out->man[a];
+  }
   return FTLE_OK;
 }
 

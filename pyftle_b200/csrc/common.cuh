@@ -26,6 +26,11 @@ struct GridK {
   double spacing[3];
   int periodic;
   long long nodes;
+  // for the FP64 path's correctly rounded division by the spacing (plain_f64.cu)
+  double rcp_hi[3], rcp_lo[3];             // 1/spacing as RN(1/s) and the rest of it
+  unsigned div_min;                        // high word of the least |x - origin| it covers
+  double man[3], man_hi[3], man_lo[3];     // spacing / 2^man_exp in +-[1, 2), its reciprocal
+  int man_exp[3];
 };
 
 int grid_from_abi(const ftle_grid *g, GridK *out);
@@ -67,14 +72,6 @@ inline unsigned grid_blocks(int64_t n, int threads, int per_sm = 8) {
 __device__ __forceinline__ int wrap_index(int q, int n) {
   int r = q % n;
   return r < 0 ? r + n : r;
-}
-
-// Node id of (i, j) / (i, j, k) in the reference's meshgrid-"xy" flattening.
-__device__ __forceinline__ long long node2(const GridK &g, int i, int j) {
-  return (long long)j * g.n[0] + i;
-}
-__device__ __forceinline__ long long node3(const GridK &g, int i, int j, int k) {
-  return ((long long)j * g.n[0] + i) * g.n[2] + k;
 }
 
 // Largest eigenvalue of a symmetric 3x3 matrix by cyclic Jacobi rotations (FP64);

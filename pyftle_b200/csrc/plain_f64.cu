@@ -22,58 +22,119 @@ namespace ftle {
 // cell location and interpolation (bit-exact with the reference)
 // ---------------------------------------------------------------------------
 
+// The cell of a point: the record of its lower corner, byte steps to the next node along
+// each axis, in-cell fractions.
 template <int DIM>
 struct Cell64 {
-  int i0[DIM], i1[DIM];
+  const char *p;
+  long long d[DIM];
   double f[DIM];
 };
 
-// (x - origin)/spacing per axis, then GridInterp.cpp's floor and "x0 >= 0 &&
-// x0+1 < n" test, written as 0 <= p < n-1 (equal for every finite p, and it
-// also rejects NaN / inf, which the reference rejects through the INT_MIN its
-// float->int conversion returns).  Periodic grids wrap the cell instead.
-template <int DIM>
-__device__ __forceinline__ bool locate64(const GridK &g, const double *x, Cell64<DIM> &c) {
-#pragma unroll
-  for (int a = 0; a < DIM; ++a) {
-    const double p = (x[a] - g.origin[a]) / g.spacing[a];
-    if (g.periodic) {
-      const double fl = floor(p);
-      if (!(fabs(fl) < 1.0e9)) return false;
-      c.f[a] = p - fl;
-      const int q = wrap_index((int)fl, g.n[a]);
-      c.i0[a] = q;
-      c.i1[a] = (q + 1 == g.n[a]) ? 0 : q + 1;
-    } else {
-      if (!(p >= 0.0 && p < (double)(g.n[a] - 1))) return false;
-      const int q = (int)floor(p);
-      c.i0[a] = q;
-      c.i1[a] = q + 1;
-      c.f[a] = p - (double)q;
-    }
+// (x - origin) / spacing per axis as IEEE division rounds it, by multiplication.  With
+// 1/s = hi + lo (hi = RN(1/s), both from the host) q0 = RN(a hi + RN(a lo)) is within half
+// an ulp plus 2^-53 ulp of a/s, r = a - q0 s is exact in an FMA, and the last FMA's
+// argument q0 + r hi differs from a/s by less than the distance of any quotient of two
+// 53-bit numbers from a rounding boundary, so it rounds as a/s does.  That needs s and a
+// away from the ends of the exponent range: the host's div_range / div_base say where, and
+// a zero, an infinity, a NaN or any other dividend outside takes the division itself (4
+// instructions instead of ~12 and a subroutine's registers; see window_f64_kernel).
+// The same division for any dividend and spacing: on mantissas in [1, 2) (man_* from the
+// host), scaled afterwards.  Zeros, infinities and NaN keep their class and sign.
+__device__ __forceinline__ double div_scaled(double v, const GridK &g, int a) {
+  const double sign = g.spacing[a] < 0.0 ? -1.0 : 1.0;
+  if (v == 0.0 || !(fabs(v) <= 1.7976931348623157e308)) return v * sign;
+  int e = -1023;
+  if (fabs(v) < 2.2250738585072014e-308) {  // subnormal
+    v *= 0x1p60;
+    e -= 60;
   }
-  return true;
+  const int hw = __double2hiint(v);
+  e += (hw >> 20) & 0x7ff;
+  const double m = __hiloint2double((hw & 0x800fffff) | 0x3ff00000, __double2loint(v));
+  const double q0 = fma(m, g.man_hi[a], m * g.man_lo[a]);
+  const double q = fma(fma(-q0, g.man[a], m), g.man_hi[a], q0);
+  e -= g.man_exp[a];
+  e = e < -1200 ? -1200 : (e > 1200 ? 1200 : e);
+  const int half = e >> 1;  // two factors inside the exponent range
+  return q * __hiloint2double((1023 + half) << 20, 0) *
+         __hiloint2double((1023 + e - half) << 20, 0);
 }
 
-// Corner node ids in the reference's operand order:
+template <int DIM>
+__device__ __forceinline__ void grid_coords(const GridK &g, const double *x, double *p) {
+  unsigned least = 0x7fffffffu;
+#pragma unroll
+  for (int a = 0; a < DIM; ++a) {
+    const double v = x[a] - g.origin[a];
+    least = min(least, (unsigned)__double2hiint(v) & 0x7fffffffu);
+    const double q0 = fma(v, g.rcp_hi[a], v * g.rcp_lo[a]);
+    p[a] = fma(fma(-q0, g.spacing[a], v), g.rcp_hi[a], q0);
+  }
+  if (least < g.div_min) {
+#pragma unroll
+    for (int a = 0; a < DIM; ++a) p[a] = div_scaled(x[a] - g.origin[a], g, a);
+  }
+}
+
+// Node stride of each axis in the meshgrid-"xy" order (2D j*nx + i, 3D (j*nx + i)*nz + k).
+template <int DIM>
+__device__ __forceinline__ long long node_stride(const GridK &g, int a) {
+  if constexpr (DIM == 2) return a == 0 ? 1 : g.n[0];
+  return a == 0 ? g.n[2] : (a == 1 ? (long long)g.n[0] * g.n[2] : 1);
+}
+
+// GridInterp.cpp's floor and "x0 >= 0 && x0+1 < n" test, equal for every finite p, which
+// also rejects NaN / inf (the reference rejects them through the INT_MIN its float->int
+// conversion returns).  Periodic grids wrap the cell instead.  Adding 1.5 * 2^52 rounding
+// down leaves floor(p) in the low word and 0x43380000 (plus its sign) in the high word for
+// |p| < 2^31: two FP64 additions in place of three conversions on the quarter-rate unit.
+// RB: bytes of a node's record at `base`.
+template <int DIM, int RB>
+__device__ __forceinline__ bool locate64(const GridK &g, const void *base, const double *x,
+                                         Cell64<DIM> &c) {
+  constexpr double kMagic = 6755399441055744.0;
+  double p[DIM];
+  grid_coords<DIM>(g, x, p);
+  bool ok = true;
+  long long node = 0;
+#pragma unroll
+  for (int a = 0; a < DIM; ++a) {
+    const double t = __dadd_rd(p[a], kMagic);
+    c.f[a] = p[a] - (t - kMagic);
+    int q = __double2loint(t);
+    const int n = g.n[a];
+    const long long stride = node_stride<DIM>(g, a);
+    c.d[a] = stride * RB;
+    if (g.periodic) {
+      ok = ok && __double2hiint(t) == 0x43380000 + (q >> 31) &&
+           (unsigned)(q + 999999999) <= 1999999998u;
+      if ((unsigned)q >= (unsigned)n) {  // usually within one period of the grid
+        q += q < 0 ? n : -n;
+        if ((unsigned)q >= (unsigned)n) q = wrap_index(q, n);
+      }
+      if (q + 1 == n) c.d[a] = -(long long)(n - 1) * stride * RB;
+    } else {
+      ok = ok && __double2hiint(t) == 0x43380000 && (unsigned)q < (unsigned)(n - 1);
+    }
+    node += q * stride;
+  }
+  c.p = static_cast<const char *>(base) + node * RB;
+  return ok;
+}
+
+// Corner records in the reference's operand order:
 //   2D v00 v10 v01 v11;  3D x0y0z0 x1y0z0 x0y0z1 x1y0z1 x0y1z0 x1y1z0 x0y1z1 x1y1z1
 template <int DIM>
-__device__ __forceinline__ void corners(const GridK &g, const Cell64<DIM> &c,
-                                        long long *nd) {
-  if constexpr (DIM == 2) {
-    nd[0] = node2(g, c.i0[0], c.i0[1]);
-    nd[1] = node2(g, c.i1[0], c.i0[1]);
-    nd[2] = node2(g, c.i0[0], c.i1[1]);
-    nd[3] = node2(g, c.i1[0], c.i1[1]);
-  } else {
-    nd[0] = node3(g, c.i0[0], c.i0[1], c.i0[2]);
-    nd[1] = node3(g, c.i1[0], c.i0[1], c.i0[2]);
-    nd[2] = node3(g, c.i0[0], c.i0[1], c.i1[2]);
-    nd[3] = node3(g, c.i1[0], c.i0[1], c.i1[2]);
-    nd[4] = node3(g, c.i0[0], c.i1[1], c.i0[2]);
-    nd[5] = node3(g, c.i1[0], c.i1[1], c.i0[2]);
-    nd[6] = node3(g, c.i0[0], c.i1[1], c.i1[2]);
-    nd[7] = node3(g, c.i1[0], c.i1[1], c.i1[2]);
+__device__ __forceinline__ void corners(const Cell64<DIM> &c, const char **r) {
+  constexpr int kSecond = DIM == 2 ? 1 : 2;  // the axis that moves second
+  r[0] = c.p;
+  r[1] = r[0] + c.d[0];
+  r[2] = r[0] + c.d[kSecond];
+  r[3] = r[1] + c.d[kSecond];
+  if constexpr (DIM == 3) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) r[4 + q] = r[q] + c.d[1];
   }
 }
 
@@ -106,19 +167,19 @@ template <int DIM>
 __device__ __forceinline__ void velocity_planar(const GridK &g, const double *__restrict__ snap,
                                                 const double *x, double *u) {
   Cell64<DIM> c;
-  if (!locate64<DIM>(g, x, c)) {
+  if (!locate64<DIM, 8>(g, snap, x, c)) {
 #pragma unroll
     for (int a = 0; a < DIM; ++a) u[a] = 0.0;
     return;
   }
-  long long nd[1 << DIM];
-  corners<DIM>(g, c, nd);
+  const char *r[1 << DIM];
+  corners<DIM>(c, r);
 #pragma unroll
   for (int comp = 0; comp < DIM; ++comp) {
-    const double *s = snap + (long long)comp * g.nodes;
     double v[1 << DIM];
 #pragma unroll
-    for (int q = 0; q < (1 << DIM); ++q) v[q] = __ldg(s + nd[q]);
+    for (int q = 0; q < (1 << DIM); ++q)
+      v[q] = __ldg(reinterpret_cast<const double *>(r[q] + comp * g.nodes * 8));
     u[comp] = interp_corners<DIM>(v, c.f);
   }
 }
@@ -127,51 +188,65 @@ __device__ __forceinline__ void velocity_planar(const GridK &g, const double *__
 // packed FP64 snapshot records: record (s, node) = [snapshot s | successor]
 // ---------------------------------------------------------------------------
 
+// The (time-blended) corner values a thread interpolated last.  RK4's third stage has the
+// time of the second and, a fraction of a cell away, nearly always its cell; so have the
+// first stage of a step and the last of the step before where t + h rounds to the next t.
+// Such a stage takes the values from here: the same bits, without the loads and the blend.
+template <int DIM>
+struct Corners64 {
+  const char *p = nullptr;  // record of the lower corner in its snapshot
+  double alpha;
+  double v[DIM][1 << DIM];
+};
+
 // HOLD: only the first half is read.  2D record = 4 doubles, 3D = 6 doubles
 // (48 bytes, so every record is 16-byte aligned).
-template <int DIM, bool BLEND>
+template <int DIM, bool BLEND, bool TRY>
 __device__ __forceinline__ void velocity_packed(const GridK &g, const double *__restrict__ rec,
-                                                double alpha, const double *x, double *u) {
+                                                double alpha, const double *x, double *u,
+                                                Corners64<DIM> &last) {
   Cell64<DIM> c;
-  if (!locate64<DIM>(g, x, c)) {
+  if (!locate64<DIM, 16 * DIM>(g, rec, x, c)) {
 #pragma unroll
     for (int a = 0; a < DIM; ++a) u[a] = 0.0;
     return;
   }
-  long long nd[1 << DIM];
-  corners<DIM>(g, c, nd);
-  double v[DIM][1 << DIM];
-  const double oma = 1.0 - alpha;
+  if (!TRY || c.p != last.p || (BLEND && alpha != last.alpha)) {
+    last.p = c.p;
+    last.alpha = alpha;
+    const char *rp[1 << DIM];
+    corners<DIM>(c, rp);
+    const double oma = 1.0 - alpha;
 #pragma unroll
-  for (int q = 0; q < (1 << DIM); ++q) {
-    const double *r = rec + nd[q] * (2 * DIM);
-    if constexpr (DIM == 2) {
+    for (int q = 0; q < (1 << DIM); ++q) {
+      const double *r = reinterpret_cast<const double *>(rp[q]);
       const double2 a = __ldg(reinterpret_cast<const double2 *>(r));
-      if constexpr (BLEND) {
-        const double2 b = __ldg(reinterpret_cast<const double2 *>(r) + 1);
-        v[0][q] = a.x * oma + b.x * alpha;
-        v[1][q] = a.y * oma + b.y * alpha;
+      if constexpr (DIM == 2) {
+        if constexpr (BLEND) {
+          const double2 b = __ldg(reinterpret_cast<const double2 *>(r) + 1);
+          last.v[0][q] = a.x * oma + b.x * alpha;
+          last.v[1][q] = a.y * oma + b.y * alpha;
+        } else {
+          last.v[0][q] = a.x;
+          last.v[1][q] = a.y;
+        }
       } else {
-        v[0][q] = a.x;
-        v[1][q] = a.y;
-      }
-    } else {
-      const double2 a = __ldg(reinterpret_cast<const double2 *>(r));
-      if constexpr (BLEND) {
-        const double2 m = __ldg(reinterpret_cast<const double2 *>(r) + 1);
-        const double2 b = __ldg(reinterpret_cast<const double2 *>(r) + 2);
-        v[0][q] = a.x * oma + m.y * alpha;
-        v[1][q] = a.y * oma + b.x * alpha;
-        v[2][q] = m.x * oma + b.y * alpha;
-      } else {
-        v[0][q] = a.x;
-        v[1][q] = a.y;
-        v[2][q] = __ldg(r + 2);
+        if constexpr (BLEND) {
+          const double2 m = __ldg(reinterpret_cast<const double2 *>(r) + 1);
+          const double2 b = __ldg(reinterpret_cast<const double2 *>(r) + 2);
+          last.v[0][q] = a.x * oma + m.y * alpha;
+          last.v[1][q] = a.y * oma + b.x * alpha;
+          last.v[2][q] = m.x * oma + b.y * alpha;
+        } else {
+          last.v[0][q] = a.x;
+          last.v[1][q] = a.y;
+          last.v[2][q] = __ldg(r + 2);
+        }
       }
     }
   }
 #pragma unroll
-  for (int comp = 0; comp < DIM; ++comp) u[comp] = interp_corners<DIM>(v[comp], c.f);
+  for (int comp = 0; comp < DIM; ++comp) u[comp] = interp_corners<DIM>(last.v[comp], c.f);
 }
 
 // ---------------------------------------------------------------------------
@@ -201,72 +276,103 @@ __device__ __forceinline__ void time_pair(const WinK &w, double t, int &s0, doub
   }
 }
 
-template <int DIM, int MODE>
-__device__ __forceinline__ void field(const WinK &w, int step, double t, const double *x,
-                                      double *u) {
+// The time lookups of a run of steps, shared by the lanes of a warp: lane PTS*k + c holds
+// point c (t, t + h/2, t + h) of step first + k, so a lookup and its two divisions run once
+// per 10 RK4 steps (32 Euler / AB2 steps) instead of once per particle and stage; a stage
+// takes its pair from the lane that holds it.
+template <int MODE, int INTEG>
+struct StepTimes {
+  static constexpr int kPoints = INTEG == FTLE_RK4 ? 3 : 1;
+  static constexpr int kSteps = 32 / kPoints;
+  int s = 0;
+  double alpha = 0.0;
+  __device__ __forceinline__ void load(const WinK &w, int first) {
+    if constexpr (MODE == FTLE_BLEND) {
+      const int lane = threadIdx.x & 31, c = lane % kPoints;
+      const double t = w.t0 + (double)(first + lane / kPoints) * w.h;
+      time_pair(w, c == 0 ? t : (c == 1 ? t + 0.5 * w.h : t + w.h), s, alpha);
+    }
+  }
+};
+
+// Velocity at point c of the k-th step of `times` (step number `step`).
+template <int DIM, bool TRY, int MODE, int INTEG>
+__device__ __forceinline__ void field(const WinK &w, const StepTimes<MODE, INTEG> &times, int k,
+                                      int step, int c, const double *x, double *u,
+                                      Corners64<DIM> &last) {
+  const double *recs = static_cast<const double *>(w.snaps);
   const long long rec_set = w.g.nodes * (2 * DIM);
   if constexpr (MODE == FTLE_HOLD) {
     int s = w.first_snapshot + step;
     if (w.periodic_time) s %= w.num_snaps;
-    velocity_packed<DIM, false>(w.g, static_cast<const double *>(w.snaps) + (long long)s * rec_set, 0.0, x, u);
+    velocity_packed<DIM, false, TRY>(w.g, recs + s * rec_set, 0.0, x, u, last);
   } else {
-    int s0;
-    double alpha;
-    time_pair(w, t, s0, alpha);
-    velocity_packed<DIM, true>(w.g, static_cast<const double *>(w.snaps) + (long long)s0 * rec_set, alpha, x, u);
+    const int lane = k * times.kPoints + c;
+    const int s = __shfl_sync(0xffffffffu, times.s, lane);
+    const double alpha = __shfl_sync(0xffffffffu, times.alpha, lane);
+    velocity_packed<DIM, true, TRY>(w.g, recs + s * rec_set, alpha, x, u, last);
   }
 }
 
-// One particle through the whole window (integrate.py restated step by step).
+// One particle through the whole window (integrate.py restated step by step).  All lanes of
+// a warp take part (the time lookups are shared).
 template <int DIM, int MODE, int INTEG>
 __device__ __forceinline__ void advect(const WinK &w, double *x) {
   const double h = w.h;
   double vprev[DIM];
-  for (int i = 0; i < w.num_steps; ++i) {
-    const double t = w.t0 + (double)i * h;
-    if constexpr (INTEG == FTLE_EULER) {
-      double v[DIM];
-      field<DIM, MODE>(w, i, t, x, v);
-#pragma unroll
-      for (int a = 0; a < DIM; ++a) x[a] = x[a] + h * v[a];
-    } else if constexpr (INTEG == FTLE_AB2) {
-      double v[DIM];
-      field<DIM, MODE>(w, i, t, x, v);
-      if (i == 0) {
+  StepTimes<MODE, INTEG> times;
+  Corners64<DIM> last;
+  for (int first = 0; first < w.num_steps; first += times.kSteps) {
+    times.load(w, first);
+    const int run = min(times.kSteps, w.num_steps - first);
+    for (int k = 0; k < run; ++k) {
+      const int i = first + k;
+      if constexpr (INTEG == FTLE_EULER) {
+        double v[DIM];
+        field<DIM, false>(w, times, k, i, 0, x, v, last);
 #pragma unroll
         for (int a = 0; a < DIM; ++a) x[a] = x[a] + h * v[a];
+      } else if constexpr (INTEG == FTLE_AB2) {
+        double v[DIM];
+        field<DIM, false>(w, times, k, i, 0, x, v, last);
+        if (i == 0) {
+#pragma unroll
+          for (int a = 0; a < DIM; ++a) x[a] = x[a] + h * v[a];
+        } else {
+#pragma unroll
+          for (int a = 0; a < DIM; ++a) x[a] = x[a] + h * (1.5 * v[a] - 0.5 * vprev[a]);
+        }
+#pragma unroll
+        for (int a = 0; a < DIM; ++a) vprev[a] = v[a];
       } else {
+        const double hh = 0.5 * h;
+        // stages 1 and 3 try the previous stage's corners in BLEND; in HOLD, where only the
+        // loads would be saved, the test cost more than they did (2D 4 %, 3D 5 % slower)
+        constexpr bool kTry = MODE == FTLE_BLEND;
+        double kv[DIM], acc[DIM], tmp[DIM];
+        field<DIM, kTry>(w, times, k, i, 0, x, kv, last);
 #pragma unroll
-        for (int a = 0; a < DIM; ++a) x[a] = x[a] + h * (1.5 * v[a] - 0.5 * vprev[a]);
+        for (int a = 0; a < DIM; ++a) {
+          acc[a] = kv[a];
+          tmp[a] = x[a] + hh * kv[a];
+        }
+        field<DIM, false>(w, times, k, i, 1, tmp, kv, last);
+#pragma unroll
+        for (int a = 0; a < DIM; ++a) {
+          acc[a] = acc[a] + 2.0 * kv[a];
+          tmp[a] = x[a] + hh * kv[a];
+        }
+        field<DIM, kTry>(w, times, k, i, 1, tmp, kv, last);
+#pragma unroll
+        for (int a = 0; a < DIM; ++a) {
+          acc[a] = acc[a] + 2.0 * kv[a];
+          tmp[a] = x[a] + h * kv[a];
+        }
+        field<DIM, false>(w, times, k, i, 2, tmp, kv, last);
+        const double h6 = h / 6.0;
+#pragma unroll
+        for (int a = 0; a < DIM; ++a) x[a] = x[a] + h6 * (acc[a] + kv[a]);
       }
-#pragma unroll
-      for (int a = 0; a < DIM; ++a) vprev[a] = v[a];
-    } else {
-      const double hh = 0.5 * h;
-      const double th = t + 0.5 * h, tf = t + h;
-      double k[DIM], acc[DIM], tmp[DIM];
-      field<DIM, MODE>(w, i, t, x, k);
-#pragma unroll
-      for (int a = 0; a < DIM; ++a) {
-        acc[a] = k[a];
-        tmp[a] = x[a] + hh * k[a];
-      }
-      field<DIM, MODE>(w, i, th, tmp, k);
-#pragma unroll
-      for (int a = 0; a < DIM; ++a) {
-        acc[a] = acc[a] + 2.0 * k[a];
-        tmp[a] = x[a] + hh * k[a];
-      }
-      field<DIM, MODE>(w, i, th, tmp, k);
-#pragma unroll
-      for (int a = 0; a < DIM; ++a) {
-        acc[a] = acc[a] + 2.0 * k[a];
-        tmp[a] = x[a] + h * k[a];
-      }
-      field<DIM, MODE>(w, i, tf, tmp, k);
-      const double h6 = h / 6.0;
-#pragma unroll
-      for (int a = 0; a < DIM; ++a) x[a] = x[a] + h6 * (acc[a] + k[a]);
     }
   }
 }
@@ -367,8 +473,28 @@ __device__ __forceinline__ double group_ftle(const double (*P)[DIM], const doubl
 // ---------------------------------------------------------------------------
 // fused window kernel: one thread per particle, G groups per block
 // ---------------------------------------------------------------------------
-template <int DIM, int MODE, int INTEG, int G>
-__device__ __forceinline__ void window_f64_body(const WinK &w) {
+// Groups per block and blocks per SM (the register budget).  The kernel is bound by the
+// latency of its FP64 chains and by L1 data wavefronts, so the budget is the largest that
+// does not spill: 3D BLEND holds 24 blended corner values, 128 registers at 15 warps per SM
+// (5 blocks of 96 threads; 6 blocks at 96 registers spill and run 1.15x slower), 2D BLEND
+// 64 registers at 32 warps (72 at 28 1.06x, unbounded 1.22x slower), 3D HOLD 80 at 24 warps,
+// 2D HOLD 48 at 40 warps (RK4; the one-stage integrators 64).  Blocks of 96 / 128 threads
+// also spread small windows over more SMs.
+// Measured against division by IEEE `/`, conversions for floor, `%` for every periodic wrap,
+// a time lookup per thread and stage and no reuse of corners: ABC 128^3, 262,080 groups, 100
+// RK4 steps BLEND 16.11 -> 9.44 ms; turbulence 512^2, 131,072 groups, 80 steps BLEND 1.63 ->
+// 0.97 ms; gyre 512 x 256, 80,000 groups, 51 steps HOLD 0.423 -> 0.336 ms.
+template <int DIM, int MODE>
+constexpr int kGroups = DIM == 2 ? 32 : (MODE == FTLE_BLEND ? 16 : 32);
+template <int DIM, int MODE, int INTEG>
+constexpr int kBlocksPerSM = DIM == 2
+                                 ? (MODE == FTLE_HOLD && INTEG == FTLE_RK4 ? 10 : 8)
+                                 : (MODE == FTLE_BLEND ? 5 : 4);
+
+template <int DIM, int MODE, int INTEG>
+__global__ void __launch_bounds__(2 * DIM * kGroups<DIM, MODE>, kBlocksPerSM<DIM, MODE, INTEG>)
+    window_f64_kernel(const WinK w) {
+  constexpr int G = kGroups<DIM, MODE>;
   constexpr int K = 2 * DIM;
   const int tid = threadIdx.x;
   // role-minor: a warp holds every neighbour of a few groups, whose gathers mostly read
@@ -377,19 +503,16 @@ __device__ __forceinline__ void window_f64_body(const WinK &w) {
   // per-particle arithmetic is the same either way
   const int role = tid % K, gl = tid / K;
   const long long g = (long long)blockIdx.x * G + gl;
+  // threads past the last group advect nothing of their own: they follow it (read only)
   const bool active = g < w.N;
-  const long long row = (long long)role * w.N + g;
+  const long long row = (long long)role * w.N + (active ? g : w.N - 1);
   double x[DIM], x0[DIM];
 #pragma unroll
-  for (int a = 0; a < DIM; ++a) x[a] = x0[a] = 0.0;
-  if (active) {
+  for (int a = 0; a < DIM; ++a) x[a] = x0[a] = w.positions[row * DIM + a];
+  advect<DIM, MODE, INTEG>(w, x);
+  if (active && !w.keep_positions) {
 #pragma unroll
-    for (int a = 0; a < DIM; ++a) x[a] = x0[a] = w.positions[row * DIM + a];
-    advect<DIM, MODE, INTEG>(w, x);
-    if (!w.keep_positions) {
-#pragma unroll
-      for (int a = 0; a < DIM; ++a) w.positions[row * DIM + a] = x[a];
-    }
+    for (int a = 0; a < DIM; ++a) w.positions[row * DIM + a] = x[a];
   }
   if (w.ftle != nullptr) {  // uniform across the block
     __shared__ double sx[K][G][DIM];
@@ -415,20 +538,6 @@ __device__ __forceinline__ void window_f64_body(const WinK &w) {
       }
     }
   }
-}
-
-template <int DIM, int MODE, int INTEG, int G>
-__global__ void __launch_bounds__(2 * DIM * G) window_f64_kernel(const WinK w) {
-  window_f64_body<DIM, MODE, INTEG, G>(w);
-}
-
-// 2D HOLD (the reference's own semantics) with the register budget of 5 blocks per SM:
-// 1.08x faster there than the compiler's own choice; the other instantiations spill at a
-// tighter budget (2D BLEND 1.14x and 3D BLEND 1.01x slower at 5 / 4 blocks), so they keep
-// theirs.
-template <int INTEG, int G>
-__global__ void __launch_bounds__(4 * G, 5) window_f64_hold2d_kernel(const WinK w) {
-  window_f64_body<2, FTLE_HOLD, INTEG, G>(w);
 }
 
 // ---------------------------------------------------------------------------
@@ -829,12 +938,9 @@ __global__ void pack_f64_kernel(const double *__restrict__ src, long long nodes,
 
 template <int DIM, int MODE, int INTEG>
 static void launch_window(const WinK &w, cudaStream_t st) {
-  constexpr int G = DIM == 2 ? 64 : 32;
+  constexpr int G = kGroups<DIM, MODE>;
   const long long blocks = (w.N + G - 1) / G;
-  if constexpr (DIM == 2 && MODE == FTLE_HOLD)
-    window_f64_hold2d_kernel<INTEG, G><<<(unsigned)blocks, 2 * DIM * G, 0, st>>>(w);
-  else
-    window_f64_kernel<DIM, MODE, INTEG, G><<<(unsigned)blocks, 2 * DIM * G, 0, st>>>(w);
+  window_f64_kernel<DIM, MODE, INTEG><<<(unsigned)blocks, 2 * DIM * G, 0, st>>>(w);
 }
 
 template <int DIM, int MODE>
