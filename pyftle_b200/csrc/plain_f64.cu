@@ -914,20 +914,47 @@ __global__ void ftle_from_positions_kernel(const double *__restrict__ pos,
 // ---------------------------------------------------------------------------
 // FP64 snapshot packing: (S, dim, nodes) -> records (S, nodes, 2*dim)
 // ---------------------------------------------------------------------------
-template <int DIM>
-__global__ void pack_f64_kernel(const double *__restrict__ src, long long nodes, int S,
-                                int periodic_time, double *dst) {
-  const long long total = nodes * S;
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
-       i += (long long)gridDim.x * blockDim.x) {
-    const int s = (int)(i / nodes);
-    const long long p = i - (long long)s * nodes;
-    const int s1 = (s + 1 < S) ? s + 1 : (periodic_time ? 0 : s);
-    double *r = dst + i * (2 * DIM);
+// One thread per node and run of R snapshots, as pack16_kernel.  A warp's 32 records of a
+// snapshot are one contiguous piece of the destination: they go through the warp's shared
+// memory so that every store covers whole sectors (8-byte stores at the record stride kept
+// the load-store unit busy: gyre 512 x 256 x 101, 202 us; now 96 us, 6.6 TB/s).
+template <int DIM, int R>
+__global__ void __launch_bounds__(256)
+    pack_f64_kernel(const double *__restrict__ src, long long nodes, int S, int periodic_time,
+                    double *dst) {
+  __shared__ double2 stage[8][32 * DIM];
+  const int lane = threadIdx.x & 31;
+  const long long p0 = blockIdx.x * 256ll + (threadIdx.x & ~31);  // the warp's first node
+  if (p0 >= nodes) return;
+  const long long p = min(p0 + lane, nodes - 1);
+  const int count = (int)min(32ll, nodes - p0) * DIM;  // 16-byte pieces of the warp's records
+  double2 *buf = stage[threadIdx.x >> 5];
+  for (int run = blockIdx.y; run * R < S; run += gridDim.y) {
+    const int s0 = run * R;
+    double v[R + 1][DIM];
 #pragma unroll
-    for (int c = 0; c < DIM; ++c) {
-      r[c] = src[((long long)s * DIM + c) * nodes + p];
-      r[DIM + c] = src[((long long)s1 * DIM + c) * nodes + p];
+    for (int r = 0; r <= R; ++r) {
+      const int s = s0 + r < S ? s0 + r : (periodic_time ? 0 : S - 1);
+#pragma unroll
+      for (int c = 0; c < DIM; ++c) v[r][c] = __ldg(src + ((long long)s * DIM + c) * nodes + p);
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      if (s0 + r >= S) break;
+      double rec[2 * DIM];
+#pragma unroll
+      for (int c = 0; c < DIM; ++c) {
+        rec[c] = v[r][c];
+        rec[DIM + c] = v[r + 1][c];
+      }
+#pragma unroll
+      for (int j = 0; j < DIM; ++j) buf[lane * DIM + j] = make_double2(rec[2 * j], rec[2 * j + 1]);
+      __syncwarp();
+      double2 *out = reinterpret_cast<double2 *>(dst) + ((long long)(s0 + r) * nodes + p0) * DIM;
+#pragma unroll
+      for (int j = 0; j < DIM; ++j)
+        if (lane + 32 * j < count) out[lane + 32 * j] = buf[lane + 32 * j];
+      __syncwarp();
     }
   }
 }
@@ -1182,9 +1209,19 @@ namespace ftle {
 
 int pack_snapshots_f64(int32_t dim, int64_t nodes, int32_t num_snapshots, int32_t periodic_time,
                        const double *src, double *dst, void *stream) {
-  const int64_t total = nodes * num_snapshots;
-  const unsigned b = grid_blocks(total, 256);
-  DIM_DISPATCH(dim, pack_f64_kernel, src, nodes, num_snapshots, periodic_time, dst);
+  cudaStream_t st = as_stream(stream);
+#define PACK(D, R)                                                                     \
+  pack_f64_kernel<D, R><<<pack_grid(nodes, num_snapshots, R), 256, 0, st>>>(src, nodes, \
+      num_snapshots, periodic_time, dst)
+  // runs of snapshots pay in 3D (128^3 x 16: 460 -> 414 us); in 2D the second read of a value
+  // comes from L2 and single snapshots are a little faster (512 x 256 x 40: 39.7 against 42.7 us)
+  if (dim == 2)
+    PACK(2, 1);
+  else if (2 * num_snapshots >= kPackRun)
+    PACK(3, kPackRun);
+  else
+    PACK(3, 1);
+#undef PACK
   return check_launch("pack_f64_kernel");
 }
 
