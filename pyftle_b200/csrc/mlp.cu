@@ -1,25 +1,29 @@
 // mlp.cu -- BF16 tensor-core (tcgen05 / TMEM) kernels of the flow-map surrogate MLP.
 //
 // GEMM: C[M x N] (+)= A[M x K] * B[N x K]^T, BF16 operands, FP32 accumulation in
-// tensor memory.  One CTA (4 warps) owns a 128 x NT tile (NT <= 128) of C:
-//   * operands are staged in shared memory as no-swizzle core matrices (8 x 16 B) by
-//     TMA (cp.async.bulk.tensor 2D boxes, 16 bytes wide, no multicast): an operand
-//     stored row-major (K contiguous) as K-major tiles, an operand stored transposed
-//     (its M/N index contiguous) as MN-major tiles with the descriptor's major bit set,
-//     so neither needs a transposition; every product of training (X W^T, dZ W, dZ^T X)
-//     and of the Jacobian tangents runs through this one kernel; rows past M (or N) lie
-//     outside the tensor maps and arrive as zeros;
-//   * one elected thread is both the TMA producer and the tensor-core issuer: a 3-stage
-//     ring with a full barrier (TMA bytes) and an empty barrier (tcgen05.commit) per
-//     stage, so chunks c+1 and c+2 are in flight while the tensor core works on chunk c;
-//     it issues tcgen05.mma (kind::f16, M = 128, N = NT, K = 16 per instruction);
-//   * the epilogue reads the accumulator back with tcgen05.ld (warp w owns TMEM
-//     lanes 32w..32w+31 = tile rows) and applies one of the fused epilogues:
-//       EPI_F32        store (or, split-K, atomically add) FP32 C
+// tensor memory; every product of training (X W^T, dZ W, dZ^T X) and of the Jacobian
+// tangents runs through this one kernel.  Persistent, one CTA of 18 warps per SM, 128 x NT
+// tiles (NT <= 128):
+//   * a producer warp brings 64-wide K chunks of both operands by TMA (no multicast) into a
+//     4-stage ring of 128-byte-swizzled tiles: rows of 64 k for an operand stored row-major
+//     (K contiguous), rows of 64 of its M/N index for one stored transposed (read MN-major
+//     through the descriptors' major bit), so neither needs a transposition; rows past M (or
+//     N) lie outside the tensor maps and arrive as zeros;
+//   * an MMA warp accumulates each tile into one of two TMEM buffers;
+//   * 16 epilogue warps drain a buffer in one read each (32 rows x 32 columns per warp),
+//     hand it back, and apply one of the fused epilogues while the next tile runs:
+//       EPI_F32        store (or, split-K, add) FP32 C
 //       EPI_BIAS_SILU  z = acc + b: store z (FP32) and h = silu(z) (BF16)
 //       EPI_DSILU      g = acc * silu'(z_in): store g (BF16), column sums of g
 //                      (the bias gradient) atomically into colsum
 //       EPI_BIAS_F32   store acc + b (FP32)
+//     Their inputs and outputs pass through 6 KB of shared memory per warp and TMA (z_in of
+//     the next tile is fetched while this one is computed; C is added by TMA reductions).
+// These layers have K = 64-384, so the kernel is bound by the bytes of its FP32
+// pre-activations and BF16 activations.  65536 x 256 x 256 on one B200, before (16-byte-wide
+// TMA boxes, a thread storing its own row, scalar atomics) and now: BIAS_SILU 94 -> 34.8 us,
+// DSILU with column sums 98 -> 36.9 us (134 MB each, 20 us at the measured copy rate), split-K
+// weight gradient 76 -> 26.6 us (event times, cold L2).
 // Every mbarrier wait is bounded; on timeout the kernel records an error in the
 // caller's error word, waits (bounded) for its copies and MMAs in flight, skips
 // the epilogue, frees its TMEM and returns.
@@ -39,7 +43,6 @@ namespace ftle {
 namespace mlp {
 
 constexpr int kTileM = 128;
-constexpr int kStages = 3;
 constexpr int kMaxNT = 128;
 
 enum { EPI_F32 = 0, EPI_BIAS_SILU = 1, EPI_DSILU = 2, EPI_BIAS_F32 = 3 };
@@ -56,152 +59,88 @@ struct Epi {
   __nv_bfloat16 *hout;   // EPI_BIAS_SILU / EPI_DSILU BF16 output
   int ldh;
   float *colsum;         // EPI_DSILU column sums (optional)
-  int accumulate;        // EPI_F32: atomically add into c
+  int accumulate;        // EPI_F32: add into c
 };
 
-// Operand staging by TMA (cp.async.bulk.tensor, no multicast: every tile is this GPU's
-// own memory).  Each operand has a 2D tensor map over its BF16 matrix; the boxes are
-// 16 bytes wide so the shared-memory tiles come out in the no-swizzle core-matrix
-// layouts the tensor core reads:
-//   K-major operand (element (r, k) at src[r*ld + k]): kChunkK/8 boxes of 8 k x R rows,
-//     tile layout [k/8][r][16 B]: core matrices 128 B apart along the rows (SBO) and
-//     R*16 B apart along K (LBO);
-//   MN-major operand (element (r, k) at src[k*ld + r]): R/8 boxes of 8 r x kChunkK k,
-//     tile layout [r/8][k][16 B]: core matrices 128 B apart along K (LBO) and
-//     kChunkK*16 B apart along the rows (SBO).
-// Rows past M (or N) lie outside the tensor map and arrive as zeros.
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap *map, int x, int y,
-                                            uint32_t mbar) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes "
-      "[%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(mbar)
-      : "memory");
-}
+constexpr int kPStages = 4;                         // TMA -> tensor-core stage ring
+constexpr int kOperandBytes = kTileM * kChunkK * 2; // one operand's part of a stage
+constexpr int kStageBytes = 2 * kOperandBytes;
+constexpr int kEpiWarps = 16;
+constexpr int kGemmThreads = 64 + 32 * kEpiWarps;   // producer warp, MMA warp, epilogue warps
+constexpr uint32_t kAccCols = 2 * kMaxNT;           // two accumulators of up to 128 columns
+// an epilogue warp's 32 x 32 tile: FP32 (128-byte rows) and BF16 (64-byte rows)
+constexpr int kStageF32 = 32 * 32 * 4, kStageB16 = 32 * 32 * 2;
+constexpr int kEpiBytes = kStageF32 + kStageB16;
+constexpr size_t kGemmSmem = (size_t)kPStages * kStageBytes + (size_t)kEpiWarps * kEpiBytes + 1024;
 
+// One operand's K chunk by TMA: K-major one box of 64 k x R rows, MN-major boxes of 64 rows x
+// 64 k (8 KB each).
 template <bool TRANS>
 __device__ __forceinline__ void tma_operand(const CUtensorMap *map, uint32_t tile, int r0, int R,
                                             int k0, uint32_t mbar) {
   if constexpr (!TRANS) {
-#pragma unroll
-    for (int j = 0; j < kChunkK / 8; ++j) tma_load_2d(tile + j * R * 16, map, k0 + 8 * j, r0, mbar);
+    tma_load_2d(tile, map, k0, r0, mbar);
   } else {
-    for (int g = 0; g < R / 8; ++g) tma_load_2d(tile + g * kChunkK * 16, map, r0 + 8 * g, k0, mbar);
+    for (int g = 0; g < R; g += 64) tma_load_2d(tile + g * kChunkK * 2, map, r0 + g, k0, mbar);
   }
 }
-
-// Descriptor of the K = 16 slice j of an operand tile with R rows (see the layouts above).
 template <bool TRANS>
-__device__ __forceinline__ uint64_t operand_desc(uint32_t tile, int R, int j) {
-  if constexpr (!TRANS) return smem_desc(tile + j * 2 * R * 16, R * 16, 128);
-  else return smem_desc(tile + j * 256, 128, kChunkK * 16);
+__device__ __forceinline__ uint32_t operand_bytes(int R) {
+  return TRANS ? (uint32_t)((R + 63) / 64 * 64 * kChunkK * 2) : (uint32_t)(R * kChunkK * 2);
 }
 
-constexpr int kPStages = 3;    // TMA -> tensor-core stage ring (2 CTAs fit an SM)
-constexpr int kEpiWarps = 8;   // epilogue warps: two per TMEM lane quarter
-constexpr int kGemmThreads = 64 + 32 * kEpiWarps;  // producer warp, MMA warp, epilogue warps
-constexpr uint32_t kAccCols = 2 * kMaxNT;          // two accumulators of up to 128 columns
-
-// Named barrier of the 128 epilogue threads (the producer and MMA warps never join it).
-__device__ __forceinline__ void epi_barrier() {
-  asm volatile("bar.sync 1, %0;" ::"n"(32 * kEpiWarps) : "memory");
+// Descriptor of the K = 16 slice j of an operand chunk (see smem_desc_sw128).
+template <bool TRANS>
+__device__ __forceinline__ uint64_t operand_desc(uint32_t tile, int j) {
+  if constexpr (!TRANS) return smem_desc_sw128(tile + j * 32, 16, 1024);
+  else return smem_desc_sw128(tile + j * 2048, 64 * kChunkK * 2, 1024);
 }
 
-// The fused epilogues on 8 consecutive columns [n, n+8) of one tile row.
-__device__ __forceinline__ void epilogue8(const Epi &epi, float *v, int row, bool row_ok, int n,
-                                          int lane, float *colsum8) {
-  if (epi.mode == EPI_F32 || epi.mode == EPI_BIAS_F32) {
-    if (epi.mode == EPI_BIAS_F32) {
+// Byte offset of 16-byte piece c of row r in a warp's FP32 / BF16 tile (TMA's 128- and
+// 64-byte swizzles; a warp's accesses to one piece of its rows are free of bank conflicts).
+__device__ __forceinline__ uint32_t f32_piece(int r, int c) { return r * 128 + ((c ^ (r & 7)) << 4); }
+__device__ __forceinline__ uint32_t b16_piece(int r, int c) {
+  return r * 64 + ((c ^ ((r >> 1) & 3)) << 4);
+}
+
+// lane's row of 32 values into the warp's BF16 tile (rounded); v becomes the rounded values
+__device__ __forceinline__ void put_b16(unsigned char *tile, int lane, const float *v) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) v[i] += epi.bias[n + i];
+  for (int c = 0; c < 4; ++c) {
+    uint32_t p[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const __nv_bfloat162 hh = __floats2bfloat162_rn(v[8 * c + 2 * i], v[8 * c + 2 * i + 1]);
+      p[i] = *reinterpret_cast<const uint32_t *>(&hh);
     }
-    if (row_ok) {
-      float *dst = epi.c + (long long)row * epi.ldc + n;
-      if (epi.accumulate) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) atomicAdd(dst + i, v[i]);
-      } else {
-        reinterpret_cast<float4 *>(dst)[0] = make_float4(v[0], v[1], v[2], v[3]);
-        reinterpret_cast<float4 *>(dst)[1] = make_float4(v[4], v[5], v[6], v[7]);
-      }
-    }
-  } else if (epi.mode == EPI_BIAS_SILU) {
-    if (row_ok) {
-      float z[8];
-      uint32_t packed[4];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) z[i] = v[i] + epi.bias[n + i];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const __nv_bfloat162 hh = __floats2bfloat162_rn(z[2 * i] * sigmoidf_(z[2 * i]),
-                                                        z[2 * i + 1] * sigmoidf_(z[2 * i + 1]));
-        packed[i] = *reinterpret_cast<const uint32_t *>(&hh);
-      }
-      *reinterpret_cast<uint4 *>(epi.hout + (long long)row * epi.ldh + n) =
-          make_uint4(packed[0], packed[1], packed[2], packed[3]);
-      if (epi.zout) {
-        float *zd = epi.zout + (long long)row * epi.ldzout + n;
-        reinterpret_cast<float4 *>(zd)[0] = make_float4(z[0], z[1], z[2], z[3]);
-        reinterpret_cast<float4 *>(zd)[1] = make_float4(z[4], z[5], z[6], z[7]);
-      }
-    }
-  } else {  // EPI_DSILU
-    float g[8];
-    if (row_ok) {
-      const float *zs = epi.zin + (long long)row * epi.ldzin + n;
-      const float4 za = reinterpret_cast<const float4 *>(zs)[0];
-      const float4 zb = reinterpret_cast<const float4 *>(zs)[1];
-      const float z[8] = {za.x, za.y, za.z, za.w, zb.x, zb.y, zb.z, zb.w};
-      uint32_t packed[4];
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const float sg = sigmoidf_(z[i]);
-        g[i] = v[i] * dsilu_from(z[i] * sg, sg);
-      }
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const __nv_bfloat162 hh = __floats2bfloat162_rn(g[2 * i], g[2 * i + 1]);
-        packed[i] = *reinterpret_cast<const uint32_t *>(&hh);
-        // the bias gradient sums the values the next GEMM consumes
-        g[2 * i] = __low2float(hh);
-        g[2 * i + 1] = __high2float(hh);
-      }
-      *reinterpret_cast<uint4 *>(epi.hout + (long long)row * epi.ldh + n) =
-          make_uint4(packed[0], packed[1], packed[2], packed[3]);
-    } else {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) g[i] = 0.0f;
-    }
-    if (colsum8) {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        float s = g[i];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xFFFFFFFFu, s, o);
-        if (lane == 0) atomicAdd(&colsum8[i], s);
-      }
-    }
+    *reinterpret_cast<uint4 *>(tile + b16_piece(lane, c)) = make_uint4(p[0], p[1], p[2], p[3]);
   }
+}
+__device__ __forceinline__ void put_f32(unsigned char *tile, int lane, const float *v) {
+#pragma unroll
+  for (int c = 0; c < 8; ++c)
+    *reinterpret_cast<float4 *>(tile + f32_piece(lane, c)) =
+        make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
 }
 
 template <bool A_T, bool B_T>
-__global__ void __launch_bounds__(kGemmThreads, 2)
+__global__ void __launch_bounds__(kGemmThreads, 1)
     gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                     int M, int N, int K, int NT, int k_per_split, int tiles_m, int splits,
+                     const __grid_constant__ CUtensorMap tmF, const __grid_constant__ CUtensorMap tmH,
+                     int M, int N, int K, int NT, int k_per_split, int tiles_n, int splits,
                      int total, Epi epi, int *err) {
-  extern __shared__ __align__(1024) unsigned char smem[];
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
   __shared__ __align__(8) unsigned long long fullb[kPStages];
   __shared__ __align__(8) unsigned long long emptyb[kPStages];
   __shared__ __align__(8) unsigned long long tfull[2];
   __shared__ __align__(8) unsigned long long tempty[2];
+  __shared__ __align__(8) unsigned long long zfull[kEpiWarps];
   __shared__ __align__(8) unsigned long long drainb;
   __shared__ uint32_t tmem_slot;
-  __shared__ volatile int s_abort;      // set by any role on a timed-out wait
-  __shared__ volatile int s_epi_abort;  // set and read by the epilogue warps only
-  __shared__ float colsum_s[kMaxNT];
-  const int tile_bytes = (kTileM + NT) * kChunkK * 2;
+  __shared__ volatile int s_abort;  // set by any role on a timed-out wait
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t smem0 = smem_u32(smem);
+  const uint32_t smem0 = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  unsigned char *smem = smem_raw + (smem0 - smem_u32(smem_raw));
 
   if (warp == 1) tmem_alloc(smem_u32(&tmem_slot), kAccCols);
   if (threadIdx.x == 0) {
@@ -213,9 +152,9 @@ __global__ void __launch_bounds__(kGemmThreads, 2)
       mbar_init(smem_u32(&tfull[b]), 1);
       mbar_init(smem_u32(&tempty[b]), kEpiWarps);
     }
+    for (int w = 0; w < kEpiWarps; ++w) mbar_init(smem_u32(&zfull[w]), 1);
     mbar_init(smem_u32(&drainb), 1);
     s_abort = 0;
-    s_epi_abort = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   fence_before_sync();
@@ -223,12 +162,12 @@ __global__ void __launch_bounds__(kGemmThreads, 2)
   fence_after_sync();
   const uint32_t tmem = tmem_slot;
 
-  // work unit u -> (k split, m tile, n tile); consecutive units share the n tile's B
+  // work unit u -> (m tile, n tile, k split); consecutive units share the m tile's A
   auto unit = [&](int u, int &m0, int &n0, int &kbeg, int &nch) {
     const int s = u % splits;
     const int t = u / splits;
-    m0 = (t % tiles_m) * kTileM;
-    n0 = (t / tiles_m) * NT;
+    m0 = (t / tiles_n) * kTileM;
+    n0 = (t % tiles_n) * NT;
     kbeg = s * k_per_split;
     const int kend = min(K, kbeg + k_per_split);
     nch = kend > kbeg ? (kend - kbeg) / kChunkK : 0;
@@ -241,6 +180,7 @@ __global__ void __launch_bounds__(kGemmThreads, 2)
   if (warp == 0) {
     // ---- TMA producer: every chunk of every unit of this CTA into the stage ring
     if (lane == 0) {
+      const uint32_t bytes = operand_bytes<A_T>(kTileM) + operand_bytes<B_T>(NT);
       int g = 0;
       for (int u = blockIdx.x; u < total && !s_abort; u += gridDim.x) {
         int m0, n0, kbeg, nch;
@@ -252,12 +192,11 @@ __global__ void __launch_bounds__(kGemmThreads, 2)
             fail();
             break;
           }
-          const uint32_t sA = smem0 + st * tile_bytes;
-          const uint32_t sB = sA + kTileM * kChunkK * 2;
+          const uint32_t sA = smem0 + st * kStageBytes;
           const uint32_t fb = smem_u32(&fullb[st]);
-          mbar_expect_tx(fb, (uint32_t)tile_bytes);
+          mbar_expect_tx(fb, bytes);
           tma_operand<A_T>(&tmA, sA, m0, kTileM, kbeg + c * kChunkK, fb);
-          tma_operand<B_T>(&tmB, sB, n0, NT, kbeg + c * kChunkK, fb);
+          tma_operand<B_T>(&tmB, sA + kOperandBytes, n0, NT, kbeg + c * kChunkK, fb);
         }
       }
       // no load may land after the shared memory is released: wait for the last ones
@@ -285,11 +224,10 @@ __global__ void __launch_bounds__(kGemmThreads, 2)
           const int st = g % kPStages;
           if (!(ok = mbar_wait(smem_u32(&fullb[st]), (uint32_t)((g / kPStages) & 1)))) break;
           fence_after_sync();
-          const uint32_t sA = smem0 + st * tile_bytes;
-          const uint32_t sB = sA + kTileM * kChunkK * 2;
+          const uint32_t sA = smem0 + st * kStageBytes;
 #pragma unroll
           for (int q = 0; q < kChunkK / 16; ++q)
-            umma(acc, operand_desc<A_T>(sA, kTileM, q), operand_desc<B_T>(sB, NT, q), idesc,
+            umma(acc, operand_desc<A_T>(sA, q), operand_desc<B_T>(sA + kOperandBytes, q), idesc,
                  (c > 0 || q > 0) ? 1u : 0u);
           umma_commit(smem_u32(&emptyb[st]));  // the stage is free once these MMAs are done
         }
@@ -304,52 +242,136 @@ __global__ void __launch_bounds__(kGemmThreads, 2)
       mbar_wait(smem_u32(&drainb), 0u);
     }
   } else {
-    // ---- epilogue warps: TMEM lanes 32q..32q+31 (q = warp % 4) are tile rows; the two
-    // warps of a lane quarter take one half of the tile's columns each
-    const int q = warp & 3;
-    const int half = (warp - 2) >> 2;
-    const int et = threadIdx.x - 64;  // 0..255 among the epilogue threads
+    // ---- epilogue warps: TMEM lanes 32q..32q+31 (q = warp % 4) are tile rows; the four
+    // warps of a lane quarter take 32 of the tile's columns each
+    const int q = warp & 3, ew = warp - 2;
+    const int c0 = 32 * (ew >> 2);
+    unsigned char *tf = smem + kPStages * kStageBytes + ew * kEpiBytes;  // FP32 tile
+    unsigned char *th = tf + kStageF32;                                  // BF16 tile
+    const uint32_t zb = smem_u32(&zfull[ew]);
+    const bool dsilu = epi.mode == EPI_DSILU;
+    // z_in of unit u into the FP32 tile (lane 0; tiles wholly outside are not touched)
+    auto mine = [&](int m0, int n0) { return n0 + c0 < N && c0 < NT && m0 + 32 * q < M; };
+    auto fetch = [&](int u) {
+      int m0, n0, kbeg, nch;
+      unit(u, m0, n0, kbeg, nch);
+      if (!mine(m0, n0)) return;
+      mbar_expect_tx(zb, kStageF32);
+      tma_load_2d(smem_u32(tf), &tmF, n0 + c0, m0 + 32 * q, zb);
+    };
+    if (dsilu && lane == 0 && (int)blockIdx.x < total) fetch(blockIdx.x);
+    float cs0 = 0.0f, cs1 = 0.0f;  // column sums of columns 2p, 2p+1 (p = lane % 16)
+    int cs_n0 = -1;
+    auto flush = [&]() {
+      if (cs_n0 >= 0) {
+        cs0 += __shfl_xor_sync(0xffffffffu, cs0, 16);
+        cs1 += __shfl_xor_sync(0xffffffffu, cs1, 16);
+        const int n = cs_n0 + c0 + 2 * (lane & 15);
+        if (lane < 16 && n < N) {  // N is even: both columns are inside
+          atomicAdd(epi.colsum + n, cs0);
+          atomicAdd(epi.colsum + n + 1, cs1);
+        }
+      }
+      cs0 = cs1 = 0.0f;
+    };
     int j = 0;
+    uint32_t zph = 0;
     for (int u = blockIdx.x; u < total; u += gridDim.x, ++j) {
       int m0, n0, kbeg, nch;
       unit(u, m0, n0, kbeg, nch);
       const int b = j & 1;
-      const bool dsum = epi.mode == EPI_DSILU && epi.colsum;
-      if (dsum) {
-        for (int i = et; i < kMaxNT; i += 32 * kEpiWarps) colsum_s[i] = 0.0f;
-        epi_barrier();
+      bool ready = mbar_wait(smem_u32(&tfull[b]), (uint32_t)((j >> 1) & 1));
+      if (!__all_sync(0xffffffffu, ready)) {
+        if (lane == 0) fail();
+        if (dsilu && mine(m0, n0)) mbar_wait(zb, zph);  // its copy in flight has landed
+        break;
       }
-      const bool ready = !s_epi_abort && mbar_wait(smem_u32(&tfull[b]), (uint32_t)((j >> 1) & 1));
-      if (!__all_sync(0xffffffffu, ready) && lane == 0) {
-        s_epi_abort = 1;
-        fail();
-      }
-      // the epilogue warps agree before any of them leaves (they share named barriers)
-      epi_barrier();
-      if (s_epi_abort) break;
       fence_after_sync();
-      const int row = m0 + 32 * q + lane;
-      const bool row_ok = row < M;
-      const uint32_t tbase = tmem + (uint32_t)(b * kMaxNT) + ((uint32_t)(32 * q) << 16);
-      const int cw = NT / 2;  // columns per warp (a multiple of 8)
-      for (int c = half * cw; c < (half + 1) * cw; c += 8) {
-        float v[8];
-        tmem_ld8(tbase + (uint32_t)c, v);
-        const int n = n0 + c;
-        if (n >= N) continue;  // uniform across the warp
-        epilogue8(epi, v, row, row_ok, n, lane, dsum ? &colsum_s[c] : nullptr);
-      }
+      const int n = n0 + c0;
+      const bool here = mine(m0, n0);
+      float v[32];
+      if (here) tmem_ld32(tmem + (uint32_t)(b * kMaxNT + c0) + ((uint32_t)(32 * q) << 16), v);
       // the accumulator is drained: the issuer may reuse it
       fence_before_sync();
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&tempty[b]));
-      if (dsum) {
-        epi_barrier();
-        for (int i = et; i < NT && n0 + i < N; i += 32 * kEpiWarps)
-          atomicAdd(epi.colsum + n0 + i, colsum_s[i]);
-        epi_barrier();
+      if (!here) {
+        if (dsilu && lane == 0 && u + (int)gridDim.x < total) fetch(u + gridDim.x);
+        continue;
+      }
+      const int x = n, y = m0 + 32 * q;
+      if (dsilu) {
+        ready = mbar_wait(zb, zph);
+        zph ^= 1u;
+        if (!__all_sync(0xffffffffu, ready)) {
+          if (lane == 0) fail();
+          break;
+        }
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          const float4 z4 = *reinterpret_cast<const float4 *>(tf + f32_piece(lane, c));
+          const float z[4] = {z4.x, z4.y, z4.z, z4.w};
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const float sg = sigmoidf_(z[i]);
+            v[4 * c + i] *= dsilu_from(z[i] * sg, sg);
+          }
+        }
+        __syncwarp();  // the tile is read: the next unit's z_in may land
+        if (lane == 0) {
+          if (u + (int)gridDim.x < total) fetch(u + gridDim.x);
+          bulk_wait_read();
+        }
+        __syncwarp();
+        put_b16(th, lane, v);
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+          tma_store_2d(&tmH, x, y, smem_u32(th));
+          bulk_commit();
+        }
+        if (epi.colsum) {
+          // the bias gradient sums the values the next GEMM consumes; rows past M are zero
+          if (cs_n0 != n0) {
+            flush();
+            cs_n0 = n0;
+          }
+          const int p = lane & 15, r0 = lane & 16;
+#pragma unroll
+          for (int r = 0; r < 16; ++r) {
+            const uint32_t w = *reinterpret_cast<const uint32_t *>(th + b16_piece(r0 + r, p >> 2) +
+                                                                   4 * (p & 3));
+            cs0 += __uint_as_float(w << 16);
+            cs1 += __uint_as_float(w & 0xffff0000u);
+          }
+        }
+      } else {
+        if (lane == 0) bulk_wait_read();
+        __syncwarp();
+        if (epi.mode != EPI_F32) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) v[i] += __ldg(epi.bias + min(n + i, N - 1));
+        }
+        if (epi.mode != EPI_BIAS_SILU || epi.zout) put_f32(tf, lane, v);
+        if (epi.mode == EPI_BIAS_SILU) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) v[i] *= sigmoidf_(v[i]);
+          put_b16(th, lane, v);
+        }
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+          if (epi.mode == EPI_F32 && epi.accumulate)
+            tma_add_2d(&tmF, x, y, smem_u32(tf));
+          else if (epi.mode != EPI_BIAS_SILU || epi.zout)
+            tma_store_2d(&tmF, x, y, smem_u32(tf));
+          if (epi.mode == EPI_BIAS_SILU) tma_store_2d(&tmH, x, y, smem_u32(th));
+          bulk_commit();
+        }
       }
     }
+    if (epi.colsum) flush();
+    if (lane == 0) bulk_wait();
   }
   fence_before_sync();
   __syncthreads();
@@ -588,38 +610,44 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
   return fn;
 }
 
-// 2D tensor map of a BF16 operand with `rows` rows (M or N) and K columns, read in the
-// boxes gemm_bf16_kernel issues: K-major (element (r, k) at src[r*ld + k]) boxes of 8 k x
-// R rows, MN-major (element (r, k) at src[k*ld + r]) boxes of 8 r x kChunkK k.
-int operand_map(CUtensorMap *map, const void *src, bool trans, int rows, int K, int ld, int R) {
+// 2D tensor map of a row-major matrix of rows x cols elements (ld elements between rows),
+// copied in boxes of box_rows x box_cols.
+int matrix_map(CUtensorMap *map, const void *src, bool f32, int rows, int cols, int ld, int box_rows,
+               int box_cols, CUtensorMapSwizzle swizzle) {
   const PFN_cuTensorMapEncodeTiled_v12000 enc = tensor_map_encoder();
   if (!enc) {
     set_error("cuTensorMapEncodeTiled is not available from the driver");
     return FTLE_ERR_CUDA;
   }
-  cuuint64_t dims[2], strides[1] = {(cuuint64_t)ld * 2};
-  cuuint32_t box[2], elem[2] = {1, 1};
-  if (!trans) {
-    dims[0] = (cuuint64_t)K;
-    dims[1] = (cuuint64_t)rows;
-    box[0] = 8;
-    box[1] = (cuuint32_t)R;
-  } else {
-    dims[0] = (cuuint64_t)rows;
-    dims[1] = (cuuint64_t)K;
-    box[0] = 8;
-    box[1] = (cuuint32_t)kChunkK;
-  }
-  const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(src), dims,
-                         strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                         CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+  const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+  const cuuint64_t strides[1] = {(cuuint64_t)ld * (f32 ? 4 : 2)};
+  const cuuint32_t box[2] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows}, elem[2] = {1, 1};
+  const CUresult r = enc(map, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16,
+                         2, const_cast<void *>(src), dims, strides, box, elem,
+                         CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
-    set_error("cuTensorMapEncodeTiled failed (%d) for a %s operand of %d x %d, ld %d", (int)r,
-              trans ? "MN-major" : "K-major", rows, K, ld);
+    set_error("cuTensorMapEncodeTiled failed (%d) for a matrix of %d x %d, ld %d", (int)r, rows, cols,
+              ld);
     return FTLE_ERR_CUDA;
   }
   return FTLE_OK;
+}
+
+// BF16 operand with `rows` rows (M or N) and K columns, in the boxes gemm_bf16_kernel issues:
+// K-major (element (r, k) at src[r*ld + k]) 64 k x R rows, MN-major (element (r, k) at
+// src[k*ld + r]) 64 rows x 64 k.
+int operand_map(CUtensorMap *map, const void *src, bool trans, int rows, int K, int ld, int R) {
+  return trans ? matrix_map(map, src, false, K, rows, ld, kChunkK, 64, CU_TENSOR_MAP_SWIZZLE_128B)
+               : matrix_map(map, src, false, rows, K, ld, R, kChunkK, CU_TENSOR_MAP_SWIZZLE_128B);
+}
+
+// The epilogue warps' 32 x 32 tiles of an FP32 / BF16 matrix.
+int f32_tile_map(CUtensorMap *map, const float *p, int M, int N, int ld) {
+  return matrix_map(map, p, true, M, N, ld, 32, 32, CU_TENSOR_MAP_SWIZZLE_128B);
+}
+int b16_tile_map(CUtensorMap *map, const __nv_bfloat16 *p, int M, int N, int ld) {
+  return matrix_map(map, p, false, M, N, ld, 32, 32, CU_TENSOR_MAP_SWIZZLE_64B);
 }
 
 int gemm_launch(const void *A, int lda, int a_trans, const void *B, int ldb, int b_trans, int M,
@@ -668,23 +696,27 @@ int gemm_launch(const void *A, int lda, int a_trans, const void *B, int ldb, int
   splits = (K + k_per_split - 1) / k_per_split;
   Epi e = epi;
   if (splits > 1) e.accumulate = 1;
-  const size_t smem = (size_t)kPStages * (kTileM + NT) * kChunkK * 2;
   const int tiles_m = (M + kTileM - 1) / kTileM, tiles_n = (N + NT - 1) / NT;
   const int total = tiles_m * tiles_n * splits;
-  const int grid = total < 2 * kNumSMs ? total : 2 * kNumSMs;  // persistent: two CTAs per SM
+  const int grid = total < kNumSMs ? total : kNumSMs;  // persistent: one CTA per SM
   cudaStream_t st = as_stream(stream);
-  CUtensorMap tmA, tmB;
+  CUtensorMap tmA, tmB, tmF, tmH;
   int rc = operand_map(&tmA, A, a_trans != 0, M, K, lda, kTileM);
-  if (rc) return rc;
-  rc = operand_map(&tmB, B, b_trans != 0, N, K, ldb, NT);
+  if (!rc) rc = operand_map(&tmB, B, b_trans != 0, N, K, ldb, NT);
+  const float *f = epi.mode == EPI_BIAS_SILU ? epi.zout : (epi.mode == EPI_DSILU ? epi.zin : epi.c);
+  const int ldf = epi.mode == EPI_BIAS_SILU ? epi.ldzout : (epi.mode == EPI_DSILU ? epi.ldzin : epi.ldc);
+  tmF = tmA;  // unused maps still have to be valid kernel arguments
+  tmH = tmA;
+  if (!rc && f) rc = f32_tile_map(&tmF, f, M, N, ldf);
+  if (!rc && epi.hout) rc = b16_tile_map(&tmH, epi.hout, M, N, epi.ldh);
   if (rc) return rc;
 #define GL(AT, BT)                                                                              \
   do {                                                                                          \
     cudaFuncSetAttribute(gemm_bf16_kernel<AT, BT>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                         (int)smem);                                                            \
+                         (int)kGemmSmem);                                                       \
     gemm_bf16_kernel<AT, BT>                                                                    \
-        <<<grid, kGemmThreads, smem, st>>>(tmA, tmB, M, N, K, NT, k_per_split, tiles_m, splits, \
-                                           total, e, error_word);                               \
+        <<<grid, kGemmThreads, kGemmSmem, st>>>(tmA, tmB, tmF, tmH, M, N, K, NT, k_per_split,   \
+                                                tiles_n, splits, total, e, error_word);         \
   } while (0)
   if (!a_trans && !b_trans)
     GL(false, false);

@@ -287,11 +287,13 @@ class FlowMapMLP:
                   ptr(ws["dY"]), self.OUT_PAD, ptr(self.grad_bias(last)), ptr(ws["loss"]), s)
         g, ldg = ws["dY"], self.OUT_PAD
         bufs = (ws["Ga"], ws["Gb"])
-        splits = max(1, min(n // 128 // 8, 74))
+        sms = torch.cuda.get_device_properties(self.device).multi_processor_count
         for l in range(last, -1, -1):
             L = self.layers[l]
             x = ws["feat"] if l == 0 else ws[f"H{l - 1}"]
-            # dW_l (out_pad x fan_in) += G^T X  (contraction over the batch)
+            # dW_l (out_pad x fan_in) += G^T X  (contraction over the batch, split so that the
+            # 128 x 128 tiles' pieces fill the SMs once)
+            splits = max(1, sms // (-(-L.out_pad // 128) * -(-L.fan_in // 128)))
             _lib.call("ftle_mlp_gemm", ptr(g), ldg, 1, ptr(x), L.fan_in, 1,
                       ptr(self.grad_weight(l)), L.fan_in, L.out_pad, L.fan_in, n, splits, 1,
                       ptr(self.err), s)

@@ -1,0 +1,95 @@
+"""The MLP GEMM's epilogues where tiles, warps' column groups and work units end."""
+
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+from oracle import mlp_oracle as mo
+
+pytestmark = pytest.mark.gpu
+
+
+def _p(t):
+    return ctypes.c_void_p(0 if t is None else t.data_ptr())
+
+
+def _call(name, *args):
+    from pyftle_b200 import _lib
+
+    _lib.call(name, *args, ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+
+
+def _bf(shape, gen, scale=1.0):
+    return (torch.randn(*shape, generator=gen) * scale).to(torch.bfloat16).cuda()
+
+
+# M: one row group, ragged tiles, more tiles than SMs; N: below, between and past a tile, with
+# the column sums' tile changing from unit to unit (three tiles on 148 SMs)
+@pytest.mark.parametrize("M,N,K", [(8, 8, 64), (136, 40, 128), (200, 96, 64), (128, 136, 192),
+                                   (1000, 384, 64), (148 * 128 + 24, 128, 64),
+                                   (60 * 128 + 8, 384, 128)])
+def test_epilogues_on_ragged_tiles(M, N, K):
+    g = torch.Generator().manual_seed(M + N + K)
+    X, W = _bf((M, K), g), _bf((N, K), g, 0.2)
+    b = (torch.randn(N, generator=g) * 0.3).cuda()
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    pad = 24  # columns past N and rows past M belong to someone else
+    acc = X.double() @ W.double().T
+    tol = (X.double().abs() @ W.double().abs().T) * K * 2.0 ** -23 + 1e-6
+
+    def out(dtype):
+        return torch.full((M + 2, N + pad), 7.0, dtype=dtype, device="cuda")
+
+    def check(t, ref, tol):
+        assert torch.all((t[:M, :N].double() - ref).abs() <= tol)
+        assert torch.all(t[M:] == 7.0) and torch.all(t[:, N:] == 7.0)
+
+    Z, H, Y = out(torch.float32), out(torch.bfloat16), out(torch.float32)
+    _call("ftle_mlp_linear", _p(X), K, _p(W), K, _p(b), M, N, K, 1, _p(Z), N + pad, _p(H), N + pad,
+          _p(err))
+    _call("ftle_mlp_linear", _p(X), K, _p(W), K, _p(b), M, N, K, 0, _p(Y), N + pad, _p(None), 0,
+          _p(err))
+    check(Z, acc + b.double(), tol)
+    assert torch.equal(Y, Z)
+    z = Z[:M, :N].double()
+    # sigma's hardware tanh is within 2^-11, the activation rounds to BF16
+    check(H, z * torch.sigmoid(z), z.abs() * 2.0 ** -10 + (z * torch.sigmoid(z)).abs() * 2.0 ** -8)
+    H2 = out(torch.bfloat16)
+    _call("ftle_mlp_linear", _p(X), K, _p(W), K, _p(b), M, N, K, 1, _p(None), 0, _p(H2), N + pad,
+          _p(err))
+    assert torch.equal(H2, H)
+
+    G, cs = out(torch.bfloat16), torch.full((N,), 0.5, device="cuda")
+    _call("ftle_mlp_gemm_dsilu", _p(X), K, 0, _p(W), K, 0, M, N, K, _p(Z), N + pad, _p(G), N + pad,
+          _p(cs), _p(err))
+    ds = torch.from_numpy(mo.dsilu(z.cpu().numpy())).cuda()
+    check(G, acc * ds, acc.abs() * (2.0 ** -9 + z.abs() * 2.0 ** -10) + (acc * ds).abs() * 2.0 ** -8
+          + tol * 2.0)
+    sums = G[:M, :N].double()
+    assert torch.all((cs.double() - 0.5 - sums.sum(0)).abs()
+                     <= (sums.abs().sum(0) + 0.5) * M * 2.0 ** -24)
+    G2 = out(torch.bfloat16)
+    _call("ftle_mlp_gemm_dsilu", _p(X), K, 0, _p(W), K, 0, M, N, K, _p(Z), N + pad, _p(G2), N + pad,
+          _p(None), _p(err))
+    assert torch.equal(G2, G)
+    torch.cuda.synchronize()
+    assert int(err.item()) == 0
+
+
+@pytest.mark.parametrize("splits", [1, 5, 148, 1000])
+@pytest.mark.parametrize("M,N", [(8, 64), (264, 136)])
+def test_split_k_adds_into_c(M, N, splits):
+    g = torch.Generator().manual_seed(splits)
+    K = 64 * 37
+    A, B = _bf((K, M), g), _bf((K, N), g)
+    C = torch.full((M + 1, N + 4), 3.0, device="cuda")
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    _call("ftle_mlp_gemm", _p(A), M, 1, _p(B), N, 1, _p(C), N + 4, M, N, K, splits, 1, _p(err))
+    ref = 3.0 + A.double().T @ B.double()
+    tol = (A.double().abs().T @ B.double().abs() + 3.0) * K * 2.0 ** -23
+    assert torch.all((C[:M, :N].double() - ref).abs() <= tol)
+    assert torch.all(C[M:] == 3.0) and torch.all(C[:, N:] == 3.0)
+    assert int(err.item()) == 0
+    assert np.isfinite(C.cpu().numpy()).all()
