@@ -67,11 +67,16 @@ class NeighboringParticles:
         self.num_neighbors = self.positions.shape[1] * 2
         assert self.positions.shape[0] % self.num_neighbors == 0, (
             f"positions.shape[0] must be a multiple of {self.num_neighbors}")
-        self.initial_delta_top_bottom = compute_delta_top_bottom(self.positions, self.num_neighbors)
-        self.initial_delta_right_left = compute_delta_right_left(self.positions, self.num_neighbors)
+        # the deltas are planes of one (dim, N, dim) block, which initial_deltas() hands out
+        roles = self.positions.view(self.num_neighbors, -1, self.dim)
+        deltas = torch.empty((self.dim,) + tuple(roles.shape[1:]), dtype=torch.float64,
+                             device=self.positions.device)
+        torch.sub(roles[1], roles[0], out=deltas[0])
+        torch.sub(roles[2::2], roles[3::2], out=deltas[1:])
+        self.initial_delta_right_left = deltas[0]
+        self.initial_delta_top_bottom = deltas[1]
         if self.positions.shape[1] == 3:
-            self.initial_delta_front_back = compute_delta_front_back(self.positions,
-                                                                     self.num_neighbors)
+            self.initial_delta_front_back = deltas[2]
         else:
             self.initial_delta_front_back = torch.zeros(0, dtype=torch.float64,
                                                         device=self.positions.device)
@@ -105,6 +110,13 @@ class NeighboringParticles:
         parts = [self.initial_delta_right_left, self.initial_delta_top_bottom]
         if self.dim == 3:
             parts.append(self.initial_delta_front_back)
+        first = parts[0]
+        size = first.numel()
+        if all(p.is_contiguous() and p.shape == first.shape
+               and p.untyped_storage().data_ptr() == first.untyped_storage().data_ptr()
+               and p.storage_offset() == first.storage_offset() + i * size
+               for i, p in enumerate(parts)):
+            return first.as_strided((self.dim,) + tuple(first.shape), (size,) + first.stride())
         return torch.stack(parts).contiguous()
 
     def positions_host(self) -> np.ndarray:
