@@ -93,3 +93,28 @@ def test_split_k_adds_into_c(M, N, splits):
     assert torch.all(C[M:] == 3.0) and torch.all(C[:, N:] == 3.0)
     assert int(err.item()) == 0
     assert np.isfinite(C.cpu().numpy()).all()
+
+
+@pytest.mark.parametrize("outs,lddy,off", [(1, 8, 0), (2, 64, 0), (4, 64, 0), (3, 64, 4), (3, 5, 0)])
+@pytest.mark.parametrize("n", [1, 9, 4099])
+def test_loss_gradient_rows(n, outs, lddy, off):
+    """Wide and single-column stores (a row length or an address that forbids the wide ones)."""
+    g = torch.Generator().manual_seed(n + outs)
+    y = torch.randn(n, lddy + 2, generator=g).cuda()
+    target = torch.randn(n, outs, generator=g).cuda()
+    buf = torch.full((off + n * lddy + 8,), 7.0, dtype=torch.bfloat16, device="cuda")
+    dy = buf[off:]
+    db, loss = torch.zeros(4, device="cuda"), torch.zeros(1, device="cuda")
+    _call("ftle_mlp_mse_grad", _p(y), lddy + 2, _p(target), outs, n, _p(dy), lddy, _p(db), _p(loss))
+    d = y[:, :outs] - target
+    got = dy[:n * lddy].view(n, lddy)
+    # one FP32 rounding per product, then BF16
+    assert torch.all((got[:, :outs].double() - 2.0 * d.double() / n).abs()
+                     <= (2.0 * d.double() / n).abs() * 2.0 ** -8)
+    assert torch.all(got[:, outs:] == 0.0) and torch.all(buf[off + n * lddy:] == 7.0)
+    assert torch.all(buf[:off] == 7.0) and torch.all(db[outs:] == 0.0)
+    sums = got[:, :outs].double()
+    assert torch.all((db[:outs].double() - sums.sum(0)).abs()
+                     <= sums.abs().sum(0) * n * 2.0 ** -24 + 1e-30)
+    assert abs(float(loss) - float(d.double().square().sum() / n)) <= n * 2.0 ** -22 * float(
+        d.double().square().sum() / n)
