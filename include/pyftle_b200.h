@@ -299,6 +299,21 @@ int ftle_mlp_jacobian_ftle3(const float *jx, const float *jy, const float *jz, i
 int ftle_mlp_apply_displacement3(const double *points, const float *y, int32_t ldy, int64_t n,
                                  double scale, double *out, void *stream);
 
+/* Fused FTLE field of a network with flat parameters (layer by layer: weights out x in, then
+ * biases; the output layer's rows padded to 64): dim 2 or 3, num_freq 32 or 64, hidden a
+ * multiple of 64 up to 384, depth 1 to 8 (shared memory permitting).
+ * ftle_mlp_field_bytes() is the packed weights' size, -1 for another shape.  points are rows
+ * (x0 .. , t0) of dim + 1 doubles, w the FP32 parameters (their biases are read), freq rows
+ * as for ftle_mlp_features / ftle_mlp_features3; ftle receives n values.  The result is that
+ * of the layered kernels (ftle_mlp_linear, ftle_mlp_gemm_dsilu, ftle_mlp_jacobian_ftle*). */
+int64_t ftle_mlp_field_bytes(int32_t dim, int32_t hidden, int32_t depth, int32_t num_freq);
+int ftle_mlp_field_pack(int32_t dim, int32_t hidden, int32_t depth, int32_t num_freq,
+                        const void *w_bf16, void *packed, void *stream);
+int ftle_mlp_field(int32_t dim, int32_t hidden, int32_t depth, int32_t num_freq,
+                   const double *points, int64_t n, const void *packed, const float *w,
+                   const float *freq, double out_scale, double T, double *ftle,
+                   int32_t *error_word, void *stream);
+
 /* Fused surrogate inference for the fixed shape 32 frequencies (64 features) ->
  * 4 x 256 SiLU -> 2 outputs: one persistent launch evaluates the network and its
  * two Jacobian tangents per seed and writes the FTLE (as ftle_mlp_jacobian_ftle)

@@ -1,10 +1,7 @@
-// umma.cuh -- tcgen05 (5th-generation tensor core) helpers shared by the MLP kernels.
+// umma.cuh -- tcgen05 (5th-generation tensor core), TMA and mbarrier helpers of the MLP kernels.
 //
-// Shared-memory operands use the no-swizzle K-major "core matrix" layout: a core
-// matrix is 8 rows x 16 bytes (8 BF16 along K) stored contiguously (128 B); within
-// a kChunkK-wide K chunk the core matrices along K are 128 B apart (the descriptor's
-// leading byte offset) and the 8-row groups kChunkK*16 B apart (its stride byte
-// offset).  One tcgen05.mma of kind::f16 consumes K = 16 (two core matrices along K).
+// Shared-memory operands are tiles of 128-byte rows (64 BF16), swizzled as TMA's SWIZZLE_128B.
+// One tcgen05.mma of kind::f16 consumes K = 16.
 #pragma once
 
 #include <cstdint>
@@ -15,19 +12,15 @@ namespace ftle {
 namespace mlp {
 
 constexpr int kChunkK = 64;
-constexpr long long kWaitLimit = 4000000;  // bounded mbarrier polls (seconds at most)
+constexpr int kWaitLimit = 200000;     // bounded mbarrier tries (seconds at most)
+constexpr uint32_t kWaitNs = 10000;
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
-// Byte offset of element (r, k) of an R x kChunkK K-major tile (no swizzle).
-__device__ __forceinline__ uint32_t kmaj_off(int r, int k) {
-  return (uint32_t)((r >> 3) * (kChunkK * 16) + (k >> 3) * 128 + (r & 7) * 16 + (k & 7) * 2);
-}
-
-// Shared-memory matrix descriptor: start address, leading (K-direction) and
-// stride (8-row direction) byte offsets in 16-byte units, version 1, no swizzle.
+// Shared-memory matrix descriptor: start address, leading and stride byte offsets in 16-byte
+// units, version 1, no swizzle.
 __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo, uint32_t sbo) {
   uint64_t d = 0;
   d |= (uint64_t)((saddr >> 4) & 0x3FFFu);
@@ -35,6 +28,12 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo, uint
   d |= (uint64_t)((sbo >> 4) & 0x3FFFu) << 32;
   d |= (uint64_t)1 << 46;
   return d;
+}
+
+// Byte offset of element (r, k) of such a tile with 128-byte rows (64 BF16), swizzled as TMA's
+// SWIZZLE_128B.
+__device__ __forceinline__ uint32_t sw128_off(int r, int k) {
+  return (uint32_t)(r * 128 + (((k >> 3) ^ (r & 7)) << 4) + (k & 7) * 2);
 }
 
 // Descriptor of an operand in 128-byte-swizzled tiles (TMA's SWIZZLE_128B, 1024-byte aligned
@@ -70,15 +69,18 @@ __device__ __forceinline__ void umma_commit(uint32_t mbar) {
       : "memory");
 }
 
+// Waits for the phase; false after kWaitLimit tries.  Each try suspends the thread for up to
+// kWaitNs: warps that poll in a tight loop take shared-memory cycles from the tensor core's
+// operand reads.
 __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity) {
-  for (long long i = 0; i < kWaitLimit; ++i) {
+  for (int i = 0; i < kWaitLimit; ++i) {
     uint32_t ok;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
         "selp.u32 %0, 1, 0, p;\n\t}\n"
         : "=r"(ok)
-        : "r"(mbar), "r"(parity)
+        : "r"(mbar), "r"(parity), "r"(kWaitNs)
         : "memory");
     if (ok) return true;
   }
@@ -206,6 +208,25 @@ __device__ __forceinline__ void tmem_ld16_start(uint32_t taddr, uint32_t (&r)[16
         "=r"(r[14]), "=r"(r[15])
       : "r"(taddr));
 }
+// 16 lanes x 2R columns in fragments (16x256b): thread t receives, for the i-th 8 columns,
+// r[4i], r[4i+1] = lane t/4, columns 2(t%4), 2(t%4)+1, and r[4i+2], r[4i+3] = lane t/4 + 8, the
+// same columns.  Valid after tmem_wait.
+__device__ __forceinline__ void tmem_ld16x256_start(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];\n"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7])
+      : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_ld16x256_start(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.16x256b.x4.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, "
+      "%11, %12, %13, %14, %15}, [%16];\n"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+        "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr));
+}
 __device__ __forceinline__ void tmem_wait16(uint32_t (&r)[16]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;\n"
                : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]),
@@ -214,6 +235,15 @@ __device__ __forceinline__ void tmem_wait16(uint32_t (&r)[16]) {
                :
                : "memory");
 }
+
+__device__ __forceinline__ void tmem_wait(uint32_t (&r)[8]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;\n"
+               : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]),
+                 "+r"(r[6]), "+r"(r[7])
+               :
+               : "memory");
+}
+__device__ __forceinline__ void tmem_wait(uint32_t (&r)[16]) { tmem_wait16(r); }
 
 }  // namespace mlp
 }  // namespace ftle

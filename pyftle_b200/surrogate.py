@@ -244,10 +244,21 @@ class FlowMapMLP:
 
     def ftle(self, points: torch.Tensor, T: float, out: Optional[torch.Tensor] = None,
              chunk: int = 1 << 20) -> torch.Tensor:
-        """FTLE (float64) of the surrogate flow map at points (n, dim+1), in chunks."""
+        """FTLE (float64) of the surrogate flow map at points (n, dim+1): one launch of the
+        fused kernel for the networks it takes, else the layered kernels in chunks."""
         n = self._check_points(points)
         if out is None:
             out = torch.empty(n, dtype=torch.float64, device=points.device)
+        shape = (self.dim, self.hidden, self.depth, self.freq.shape[0])
+        nbytes = _lib.load().ftle_mlp_field_bytes(*shape) if self.outs == self.dim else -1
+        if nbytes > 0:
+            # the weights are packed on every call: they may have changed since the last one
+            packed = torch.empty(nbytes, dtype=torch.uint8, device=self.device)
+            _lib.call("ftle_mlp_field_pack", *shape, ptr(self.wb), ptr(packed), stream_ptr())
+            _lib.call("ftle_mlp_field", *shape, ptr(points), n, ptr(packed), ptr(self.w),
+                      ptr(self.freq), self.out_scale, float(T), ptr(out), ptr(self.err),
+                      stream_ptr())
+            return out
         for i in range(0, n, chunk):
             j = min(n, i + chunk)
             _, *J = self.predict(points[i:j], jacobian=True)

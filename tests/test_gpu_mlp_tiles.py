@@ -118,3 +118,53 @@ def test_loss_gradient_rows(n, outs, lddy, off):
                      <= sums.abs().sum(0) * n * 2.0 ** -24 + 1e-30)
     assert abs(float(loss) - float(d.double().square().sum() / n)) <= n * 2.0 ** -22 * float(
         d.double().square().sum() / n)
+
+
+def _layered_ftle(net, points, T):
+    """The network's FTLE through the layered kernels."""
+    _, *jac = net.predict(points, jacobian=True)
+    out = torch.empty(points.shape[0], dtype=torch.float64, device="cuda")
+    name = "ftle_mlp_jacobian_ftle" if net.dim == 2 else "ftle_mlp_jacobian_ftle3"
+    _call(name, *(_p(j) for j in jac), net.OUT_PAD, points.shape[0], ctypes.c_double(net.out_scale),
+          ctypes.c_double(T), _p(out))
+    return out
+
+
+# one CTA or two per SM, halves of N = 160 / 192, odd 16-column steps, two feature chunks,
+# features wider than the layers, the shallowest and the deepest; tiles are 40 and 32 seeds
+@pytest.mark.parametrize("hidden,depth,freqs", [(64, 1, 32), (64, 3, 64), (128, 4, 32), (192, 2, 64),
+                                                (256, 4, 32), (256, 8, 32), (320, 2, 32),
+                                                (384, 4, 32), (384, 3, 64)])
+@pytest.mark.parametrize("dim,n", [(2, 8), (2, 4104), (3, 8), (3, 4104), (2, 20000), (3, 20000)])
+def test_fused_field_equals_the_layered_kernels(dim, n, hidden, depth, freqs):
+    from pyftle_b200.surrogate import FlowMapMLP, fourier_frequencies
+
+    net = FlowMapMLP(fourier_frequencies(freqs, dim=dim, seed=1), hidden=hidden, depth=depth,
+                     out_scale=0.2, seed=2)
+    g = torch.Generator(device="cuda").manual_seed(n)
+    for l in range(depth + 1):
+        net.bias(l)[:net.layers[l].fan_out].normal_(0.0, 0.1, generator=g)
+    pts = 6.0 * torch.rand(n, dim + 1, generator=g, dtype=torch.float64, device="cuda")
+    ref = _layered_ftle(net, pts, 2.5)
+    got = net.ftle(pts, 2.5)
+    net.check_errors()
+    # the same products in the same order and the same roundings; FP64 at the end
+    assert torch.all((got - ref).abs() <= 1e-12 + 1e-9 * ref.abs())
+    # changed weights are seen by the next call
+    net.wb.mul_(0.5)
+    assert torch.all((net.ftle(pts, 2.5) - _layered_ftle(net, pts, 2.5)).abs()
+                     <= 1e-12 + 1e-9 * ref.abs().max())
+
+
+def test_networks_the_fused_field_does_not_take_stay_layered():
+    from pyftle_b200 import _lib
+    from pyftle_b200.surrogate import FlowMapMLP, fourier_frequencies
+
+    size = _lib.load().ftle_mlp_field_bytes
+    for shape in ((2, 448, 4, 32), (2, 512, 4, 32), (3, 256, 9, 32), (2, 256, 4, 96), (4, 256, 4, 32),
+                  (2, 96, 4, 32), (2, 256, 0, 32)):
+        assert size(*shape) == -1
+    assert size(2, 256, 4, 32) == 425984 + 8192
+    net = FlowMapMLP(fourier_frequencies(32, dim=3, seed=1), hidden=512, depth=2, out_scale=0.2)
+    pts = torch.rand(64, 4, dtype=torch.float64, device="cuda")
+    assert torch.equal(net.ftle(pts, 1.0), _layered_ftle(net, pts, 1.0))
