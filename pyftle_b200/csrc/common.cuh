@@ -65,9 +65,8 @@ inline unsigned grid_blocks(int64_t n, int threads, int per_sm = 8) {
 }
 
 // Grid of a packing kernel: blocks of 256 nodes x runs of `run` snapshots per thread.  A run
-// reads (and encodes) its values once plus a successor, a single snapshot twice; series
-// shorter than half a run waste its loads.
-constexpr int kPackRun = 8;
+// reads (and encodes) its values once plus a successor, a single snapshot twice; long runs
+// take registers and leave a longer tail.
 inline dim3 pack_grid(int64_t nodes, int32_t num_snapshots, int run) {
   const int64_t runs = (num_snapshots + run - 1) / run;
   return dim3((unsigned)((nodes + 255) / 256), (unsigned)(runs < 65535 ? runs : 65535));

@@ -312,11 +312,13 @@ static int pack16(int64_t nodes, int32_t S, int32_t periodic_time, const double 
     else
       fx16_finalize_kernel<<<1, 32, 0, st>>>(h, DIM);
   }
-  // runs halve the encoding (512 x 256 x 16 to FX16: 19.8 -> 9.9 us), but not for a series of
-  // two (128^3: 89 us against 55 us)
-  if (2 * S >= kPackRun)
-    pack16_kernel<DIM, STORAGE, kPackRun>
-        <<<pack_grid(nodes, S, kPackRun), 256, 0, st>>>(src, nodes, S, periodic_time, h, recs);
+  // The fixed-point encodings cost more than the reads: runs of 8 (128^3 x 32: FX16 696 us with
+  // the range pass, 898 with runs of 2; not for a series of two, 89 us against 55).  FP16 and
+  // BF16 are two instructions: runs of 2 (700 x 700 x 60: 112 us, runs of 8 154, none 179).
+  constexpr int kRun = STORAGE == FTLE_FX15 || STORAGE == FTLE_FX16 ? 8 : 2;
+  if (2 * S >= kRun)
+    pack16_kernel<DIM, STORAGE, kRun>
+        <<<pack_grid(nodes, S, kRun), 256, 0, st>>>(src, nodes, S, periodic_time, h, recs);
   else
     pack16_kernel<DIM, STORAGE, 1>
         <<<pack_grid(nodes, S, 1), 256, 0, st>>>(src, nodes, S, periodic_time, h, recs);

@@ -1280,12 +1280,13 @@ int pack_snapshots_f64(int32_t dim, int64_t nodes, int32_t num_snapshots, int32_
 #define PACK(D, R)                                                                     \
   pack_f64_kernel<D, R><<<pack_grid(nodes, num_snapshots, R), 256, 0, st>>>(src, nodes, \
       num_snapshots, periodic_time, dst)
-  // runs of snapshots pay in 3D (128^3 x 16: 460 -> 414 us); in 2D the second read of a value
-  // comes from L2 and single snapshots are a little faster (512 x 256 x 40: 39.7 against 42.7 us)
+  // runs of snapshots pay in 3D (128^3 x 16: none 460 us, runs of 8 417, of 4 384); in 2D the
+  // second read of a value comes from L2 and single snapshots are a little faster (512 x 256
+  // x 40: 39.7 us against 42.7 with runs of 8)
   if (dim == 2)
     PACK(2, 1);
-  else if (2 * num_snapshots >= kPackRun)
-    PACK(3, kPackRun);
+  else if (num_snapshots >= 2)
+    PACK(3, 4);
   else
     PACK(3, 1);
 #undef PACK
