@@ -132,6 +132,11 @@ int ftle_ab2_update(double *x, double h, const double *v, const double *v_prev, 
 int ftle_rk4_update(double *x, double h, const double *k1, const double *k2, const double *k3,
                     const double *k4, int64_t n, void *stream);
 
+/* Initial separations and centroid of every group in one pass (particles.py:85-100, 225-237):
+ * deltas (dim, N, dim) as below, centroid (N, dim) = sum of the roles in order / (2 dim). */
+int ftle_group_init(int32_t dim, const double *positions, int64_t num_groups, double *deltas,
+                    double *centroid, void *stream);
+
 /* ---- FTLE building blocks (cauchy_green.py, ftle.py) ---------------------
  * initial_deltas: (dim, N, dim) = [right-left; top-bottom (; front-back)] at
  * t0 (particles.py:85-100); only the diagonal entries are used

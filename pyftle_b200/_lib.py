@@ -69,6 +69,7 @@ SIGNATURES = {
     "ftle_axpy": (ctypes.c_int, [_c_dp, _c_dp, _f64, _c_dp, _i64, _c_dp]),
     "ftle_ab2_update": (ctypes.c_int, [_c_dp, _f64, _c_dp, _c_dp, _i64, _c_dp]),
     "ftle_rk4_update": (ctypes.c_int, [_c_dp, _f64, _c_dp, _c_dp, _c_dp, _c_dp, _i64, _c_dp]),
+    "ftle_group_init": (ctypes.c_int, [_i32, _c_dp, _i64, _c_dp, _c_dp, _c_dp]),
     "ftle_flow_map_jacobian": (ctypes.c_int, [_i32, _c_dp, _c_dp, _i64, _c_dp, _c_dp]),
     "ftle_cauchy_green": (ctypes.c_int, [_i32, _c_dp, _i64, _c_dp, _c_dp]),
     "ftle_max_eigenvalue": (ctypes.c_int, [_i32, _c_dp, _i64, _c_dp, _c_dp]),

@@ -959,6 +959,27 @@ __global__ void ftle_from_jacobian_kernel(const double *__restrict__ J, long lon
   });
 }
 
+// Initial separations (DIM planes of N x DIM, right-left, top-bottom (, front-back)) and the
+// centroid, summed in role order, of every group: every role's rows are one contiguous block,
+// so thread e takes element e of each.
+template <int DIM>
+__global__ void group_init_kernel(const double *__restrict__ pos, long long N, double *deltas,
+                                  double *centroid) {
+  const long long n = N * DIM;
+  for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n;
+       e += (long long)gridDim.x * blockDim.x) {
+    double x[2 * DIM];
+#pragma unroll
+    for (int r = 0; r < 2 * DIM; ++r) x[r] = __ldg(pos + r * n + e);
+#pragma unroll
+    for (int j = 0; j < DIM; ++j) deltas[j * n + e] = x[plus_role(j)] - x[minus_role(j)];
+    double s = x[0];
+#pragma unroll
+    for (int r = 1; r < 2 * DIM; ++r) s = s + x[r];
+    centroid[e] = s / (double)(2 * DIM);
+  }
+}
+
 template <int DIM>
 __global__ void ftle_from_positions_kernel(const double *__restrict__ pos,
                                            const double *__restrict__ idl, long long N,
@@ -1173,6 +1194,17 @@ int ftle_rk4_update(double *x, double h, const double *k1, const double *k2, con
       KERNEL<3><<<b, THREADS, 0, as_stream(stream)>>>(__VA_ARGS__); \
   } while (0)
 constexpr int kTileThreads = 32 * kTileWarps;
+
+int ftle_group_init(int32_t dim, const double *positions, int64_t num_groups, double *deltas,
+                    double *centroid, void *stream) {
+  if (dim != 2 && dim != 3) return fail_invalid("dim must be 2 or 3");
+  if (num_groups < 0) return fail_invalid("num_groups must be >= 0");
+  if (num_groups == 0) return FTLE_OK;
+  if (!positions || !deltas || !centroid) return fail_invalid("null pointer");
+  const unsigned b = grid_blocks(num_groups * dim, 256);
+  DIM_DISPATCH(dim, group_init_kernel, 256, positions, num_groups, deltas, centroid);
+  return check_launch("group_init_kernel");
+}
 
 int ftle_flow_map_jacobian(int32_t dim, const double *positions, const double *initial_deltas,
                            int64_t num_groups, double *jacobian, void *stream) {

@@ -19,7 +19,8 @@ from dataclasses import dataclass, field
 import numpy as np
 import torch
 
-from pyftle_b200._device import as_device_f64, to_host
+from pyftle_b200 import _lib
+from pyftle_b200._device import as_device_f64, ptr, stream_ptr, to_host
 
 
 def _split(positions: torch.Tensor, num_neighbors: int):
@@ -67,20 +68,21 @@ class NeighboringParticles:
         self.num_neighbors = self.positions.shape[1] * 2
         assert self.positions.shape[0] % self.num_neighbors == 0, (
             f"positions.shape[0] must be a multiple of {self.num_neighbors}")
-        # the deltas are planes of one (dim, N, dim) block, which initial_deltas() hands out
-        roles = self.positions.view(self.num_neighbors, -1, self.dim)
-        deltas = torch.empty((self.dim,) + tuple(roles.shape[1:]), dtype=torch.float64,
-                             device=self.positions.device)
-        torch.sub(roles[1], roles[0], out=deltas[0])
-        torch.sub(roles[2::2], roles[3::2], out=deltas[1:])
-        self.initial_delta_right_left = deltas[0]
-        self.initial_delta_top_bottom = deltas[1]
-        if self.positions.shape[1] == 3:
-            self.initial_delta_front_back = deltas[2]
+        # one launch for the separations (planes of a (dim, N, dim) block, which
+        # initial_deltas() hands out) and the centroid
+        dim, dev = self.dim, self.positions.device
+        n = self.positions.shape[0] // self.num_neighbors
+        block = torch.empty((dim + 1, n, dim), dtype=torch.float64, device=dev)
+        _lib.call("ftle_group_init", dim, ptr(self.positions), n, ptr(block), ptr(block[dim]),
+                  stream_ptr())
+        planes = block.unbind()
+        self.initial_delta_right_left = planes[0]
+        self.initial_delta_top_bottom = planes[1]
+        if dim == 3:
+            self.initial_delta_front_back = planes[2]
         else:
-            self.initial_delta_front_back = torch.zeros(0, dtype=torch.float64,
-                                                        device=self.positions.device)
-        self.initial_centroid = compute_centroid(self.positions, self.num_neighbors)
+            self.initial_delta_front_back = torch.zeros(0, dtype=torch.float64, device=dev)
+        self.initial_centroid = planes[dim]
 
     def __len__(self) -> int:
         return self.positions.shape[0] // self.num_neighbors
