@@ -8,6 +8,10 @@ import numpy as np
 import torch
 
 
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (
+    lambda device: torch.cuda.current_stream(device).cuda_stream)
+
+
 def require_cuda() -> torch.device:
     if not torch.cuda.is_available():
         raise RuntimeError("pyftle_b200 needs a CUDA device (sm_100a); none is visible")
@@ -16,6 +20,9 @@ def require_cuda() -> torch.device:
 
 def as_device_f64(x, *, copy: bool = False) -> torch.Tensor:
     """Contiguous float64 CUDA tensor holding x (numpy array, sequence or tensor)."""
+    if (isinstance(x, torch.Tensor) and x.is_cuda and not copy and x.dtype == torch.float64
+            and x.is_contiguous() and x.get_device() == torch.cuda.current_device()):
+        return x
     dev = require_cuda()
     if isinstance(x, torch.Tensor):
         pinned = (not x.is_cuda) and x.is_pinned()
@@ -38,5 +45,7 @@ def ptr(t: torch.Tensor | None) -> ctypes.c_void_p:
 
 
 def stream_ptr(stream: torch.cuda.Stream | None = None) -> ctypes.c_void_p:
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return ctypes.c_void_p(s.cuda_stream)
+    if stream is None:
+        # the handle itself: a Stream object costs as much as a launch
+        return ctypes.c_void_p(_raw_stream(torch.cuda.current_device()))
+    return ctypes.c_void_p(stream.cuda_stream)

@@ -157,7 +157,7 @@ def load(path: str = LIB_PATH) -> ctypes.CDLL:
 
 def call(name: str, *args) -> int:
     """Call an entry point and raise FTLEError on a non-zero status."""
-    lib = load()
+    lib = _lib or load()
     rc = getattr(lib, name)(*args)
     if rc != FTLE_OK:
         msg = lib.ftle_last_error()

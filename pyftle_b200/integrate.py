@@ -60,8 +60,8 @@ class Integrator(ABC):
         if it.grid is None or it.snapshot is None:
             raise AssertionError("interpolator was not initialised with update(velocities, points)")
         pos = particles.positions
-        _lib.call("ftle_grid_step", it.grid.to_abi(), ptr(it.snapshot), code, float(h), ptr(pos),
-                  pos.shape[0], ptr(history), int(history_valid), stream_ptr())
+        _lib.call("ftle_grid_step", it.grid.abi, it.snapshot.data_ptr(), code, float(h),
+                  pos.data_ptr(), pos.shape[0], ptr(history), int(history_valid), stream_ptr())
         return True
 
 

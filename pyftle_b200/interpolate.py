@@ -26,8 +26,10 @@ meshgrid-"xy" layout for every shape (the reference is only right for
 
 from __future__ import annotations
 
+import math
 from abc import ABC, abstractmethod
 from dataclasses import dataclass
+from functools import cached_property
 from typing import Callable, Optional
 
 import numpy as np
@@ -35,6 +37,15 @@ import torch
 
 from pyftle_b200 import _lib
 from pyftle_b200._device import as_device_f64, ptr, require_cuda, stream_ptr, to_host
+
+
+def _extent(x: np.ndarray):
+    """(min, max) of a coordinate array, in one threaded pass where torch can read it."""
+    if x.dtype == np.float64 and x.flags.writeable and x.flags.aligned and x.size \
+            and all(s > 0 for s in x.strides):
+        lo, hi = torch.aminmax(torch.from_numpy(x))
+        return np.float64(lo.item()), np.float64(hi.item())
+    return np.min(x), np.max(x)
 
 
 @dataclass(frozen=True)
@@ -50,9 +61,14 @@ class GridSpec:
     def dim(self) -> int:
         return len(self.shape)
 
-    @property
+    @cached_property
     def nodes(self) -> int:
         return int(np.prod(self.shape))
+
+    @cached_property
+    def abi(self) -> _lib.FtleGrid:
+        """The grid's C-ABI struct, made once; for calls that only read it."""
+        return self.to_abi()
 
     @classmethod
     def from_points(cls, points, grid_shape, periodic: bool = False) -> "GridSpec":
@@ -63,7 +79,7 @@ class GridSpec:
             raise ValueError(f"points must have shape ({dim}, nodes)")
         origin, spacing = [], []
         for a in range(dim):
-            ax = np.linspace(np.min(pts[a]), np.max(pts[a]), grid_shape[a])
+            ax = np.linspace(*_extent(pts[a]), grid_shape[a])
             origin.append(float(ax[0]))
             spacing.append(float((ax[-1] - ax[0]) / (ax.shape[0] - 1)))
         return cls(tuple(int(n) for n in grid_shape), tuple(origin), tuple(spacing), periodic)
@@ -110,11 +126,10 @@ class HighPerfInterpolator(Interpolator):
         self.snapshot: Optional[torch.Tensor] = None  # (dim, nodes) float64 on the device
 
     def update(self, velocities, points=None) -> None:
-        dim = len(self.grid_shape)
         vel = as_device_f64(velocities)
-        if vel.ndim != 2 or vel.shape[0] != dim or vel.shape[1] != int(np.prod(self.grid_shape)):
-            raise ValueError(
-                f"velocities must have shape ({dim}, {int(np.prod(self.grid_shape))})")
+        shape = (len(self.grid_shape), math.prod(self.grid_shape))
+        if vel.shape != shape:
+            raise ValueError(f"velocities must have shape {shape}")
         self.velocities = vel
         self.snapshot = vel
         if points is not None:
@@ -132,8 +147,7 @@ class HighPerfInterpolator(Interpolator):
             raise ValueError(f"Unsupported point dimension: {pts.shape[-1]}")
         if out is None:
             out = torch.empty_like(pts)
-        g = self.grid.to_abi()
-        _lib.call("ftle_grid_interpolate", g, ptr(self.snapshot), ptr(pts), pts.shape[0], ptr(out),
+        _lib.call("ftle_grid_interpolate", self.grid.abi, ptr(self.snapshot), ptr(pts), pts.shape[0], ptr(out),
                   stream_ptr())
         return out
 

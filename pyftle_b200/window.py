@@ -96,7 +96,7 @@ def window_descriptor(series: SnapshotSeries, positions: torch.Tensor, ftle: Opt
             raise ValueError(f"ftle must be a contiguous float64 tensor of {n} elements on "
                              f"{positions.device}")
     w = _lib.FtleWindow()
-    w.grid = series.grid.to_abi()
+    w.grid = series.grid.abi
     w.snapshots = series.packed.data_ptr()
     w.num_snapshots = series.num_snapshots
     w.storage = series.storage
