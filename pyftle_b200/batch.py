@@ -78,7 +78,7 @@ class JudgeReport:
 
 @dataclass(frozen=True)
 class Schedule:
-    ctas_per_sm: int = 4  # the kernel fits 4 blocks of 128 threads per SM
+    ctas_per_sm: int = 4  # 4 fill the chip (in 2D a pair of blocks each)
     order: int = 1  # 1: longest windows first, 2: by start of the time range, 0: as given
 
 
@@ -340,9 +340,8 @@ class WindowBatch:
         if use_cache and self.shape_key in cache:
             self.schedule = Schedule(**cache[self.shape_key]["schedule"])
             return self.schedule
-        # blocks per SM the kernel can keep resident: 4 in 3D, up to 8 in 2D
-        ctas = (1, 2, 3, 4) if self.series.grid.dim == 3 else (2, 4, 6, 8)
-        cands = list(candidates) if candidates else [Schedule(c, o) for c in ctas
+        # 4 blocks (2D: pairs of blocks) per SM fill the chip
+        cands = list(candidates) if candidates else [Schedule(c, o) for c in (1, 2, 3, 4)
                                                      for o in (1, 2, 0)]
         timings = []
         for sch in cands:
