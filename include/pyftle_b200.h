@@ -226,6 +226,13 @@ int ftle_analytic_window_run(const ftle_flow *flow, int32_t integrator, double t
 int64_t ftle_windows_plan_bytes(const ftle_window *windows, int32_t count);
 int ftle_windows_plan(const ftle_window *windows, int32_t count, int32_t order,
                       void *host_plan, int64_t plan_bytes);
+/* As ftle_windows_plan, with the order in which window i's groups are taken: group_orders[i]
+ * is a device array of its num_groups group indices (a permutation, read by every run), or
+ * NULL for the given order.  Neighbours in that order share work items, so a spatial order
+ * makes their gathers share cache lines; positions and FTLE stay in the caller's order. */
+int ftle_windows_plan_ordered(const ftle_window *windows, int32_t count, int32_t order,
+                              const int64_t *const *group_orders, void *host_plan,
+                              int64_t plan_bytes);
 int ftle_windows_run_mixed(const ftle_window *windows, int32_t count, void *device_plan,
                            int64_t plan_bytes, int32_t ctas_per_sm, void *stream);
 

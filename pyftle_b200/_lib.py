@@ -91,6 +91,8 @@ SIGNATURES = {
                                                 _i32, _c_dp, _i64, _f64, _c_dp, _c_dp]),
     "ftle_windows_plan_bytes": (ctypes.c_int64, [ctypes.POINTER(FtleWindow), _i32]),
     "ftle_windows_plan": (ctypes.c_int, [ctypes.POINTER(FtleWindow), _i32, _i32, _c_dp, _i64]),
+    "ftle_windows_plan_ordered": (ctypes.c_int, [ctypes.POINTER(FtleWindow), _i32, _i32,
+                                                 ctypes.POINTER(_c_dp), _c_dp, _i64]),
     "ftle_windows_run_mixed": (ctypes.c_int, [ctypes.POINTER(FtleWindow), _i32, _c_dp, _i64,
                                               _i32, _c_dp]),
     # flow-map surrogate MLP (BF16 tensor-core kernels)

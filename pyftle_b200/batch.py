@@ -10,12 +10,15 @@ take work items (128 groups of one window) from a counter, longest windows first
 ``WindowBatch`` builds the plan once (``ftle_windows_plan``), keeps it on the
 device, and runs it directly or as a captured CUDA graph (``capture()`` /
 ``replay()``).  A persistent work item keeps its 128 groups for the whole window (the
-single-window path re-sorts between chunks instead), so by default the batch hands the
-kernel each seed buffer in Morton order of the groups' initial centroids: a work item
-then holds a compact patch of the domain and its gathers share cache lines.  Each run
-gathers the seeds into that order, runs the kernel, and scatters FTLE (and the final
-positions of windows that update them) back to the caller's order; per-group results
-are the same bits in either order.  ``autotune()`` times the schedule candidates (CTAs per SM,
+single-window path re-sorts between chunks instead), so by default the kernel takes each
+window's groups in Morton order of their initial centroids: a work item then holds a
+compact patch of the domain and its gathers share cache lines.  The kernel reads and
+writes the caller's buffers through the order; where windows share a buffer that one of
+them writes, or a window's buffers were exchanged, each run instead gathers the seeds
+into that order, and scatters FTLE and final positions back window by window.  Without
+the copies' launches (two a window) 40 windows of 300 groups take 0.53 ms instead of
+0.96 ms, and the 2D turbulence batch of 24 windows 16.2 ms instead of 16.6 ms.  Per-group results are the same bits in either
+order.  ``autotune()`` times the schedule candidates (CTAs per SM,
 ordering) on the batch itself and keeps the fastest; results are cached per
 batch shape in ``~/.cache/pyftle_b200/tuning.json``.
 """
@@ -110,6 +113,25 @@ def morton_order(positions: torch.Tensor, grid) -> torch.Tensor:
     return torch.argsort(key, stable=True)
 
 
+def _writes_overlap(windows: Sequence[WindowSpecRun]) -> bool:
+    """Whether a buffer that one window writes (its FTLE, or the positions that it updates)
+    overlaps a buffer that another window reads or writes."""
+    spans = []  # (first byte, end, written)
+    for w in windows:
+        for t, written in ((w.positions, not w.keep_positions), (w.ftle, True)):
+            if t.numel():
+                spans.append((t.data_ptr(), t.data_ptr() + 8 * t.numel(), written))
+    read_end = write_end = 0  # the furthest ends of the spans before
+    for first, end, written in sorted(spans):
+        if first < write_end or (written and first < read_end):
+            return True
+        if written:
+            write_end = max(write_end, end)
+        else:
+            read_end = max(read_end, end)
+    return False
+
+
 class WindowBatch:
     def __init__(self, series: SnapshotSeries, windows: Sequence[WindowSpecRun], *,
                  integrator: str = "rk4", time_mode: str = "blend",
@@ -123,15 +145,13 @@ class WindowBatch:
                        snapshot_dt=snapshot_dt)
         dim = series.grid.dim
         K = 2 * dim
-        # Spatial order: one permuted copy per distinct seed buffer (windows sharing
-        # read-only seeds share it), one FTLE buffer per window in that order.
+        # Spatial order: one permutation per distinct seed buffer (windows sharing read-only
+        # seeds share it).
         self.spatial_order = bool(spatial_order)
         self._src: List[torch.Tensor] = []      # caller's seed buffers
         self._perm: List[torch.Tensor] = []     # group permutation per buffer
-        self._sorted: List[torch.Tensor] = []   # seeds in Morton order
         self._shared: List[bool] = []          # buffer is read-only seeds (shareable)
         self._win_src: List[int] = []
-        self._win_ftle: List[torch.Tensor] = []
         for w in self.windows:
             p = w.positions
             if (p.dtype != torch.float64 or not p.is_cuda or not p.is_contiguous()
@@ -157,16 +177,11 @@ class WindowBatch:
                 self._shared.append(bool(w.keep_positions))
                 perm = morton_order(w.positions, series.grid)
                 self._perm.append(perm)
-                self._sorted.append(torch.empty_like(w.positions))
                 k = len(self._src) - 1
             self._win_src.append(k)
-            self._win_ftle.append(torch.empty_like(w.ftle))
-        self._gather()
-        arr = (_lib.FtleWindow * len(self.windows))()
+        self.count = len(self.windows)
         self._map_period: List[float] = []
-        for i, w in enumerate(self.windows):
-            pos = self._sorted[self._win_src[i]] if self.spatial_order else w.positions
-            ftle = self._win_ftle[i] if self.spatial_order else w.ftle
+        for w in self.windows:
             if w.map_period is not None:
                 mp = w.map_period
             elif time_mode == "hold":  # the reference's T = (p - 1)|dt| (ftle_solver.py:156)
@@ -174,28 +189,51 @@ class WindowBatch:
             else:
                 mp = w.num_steps * abs(w.h)
             self._map_period.append(mp)
-            arr[i] = window_descriptor(series, pos, ftle, h=w.h, num_steps=w.num_steps,
-                                       map_period=mp, t0=w.t0, first_snapshot=w.first_snapshot,
-                                       keep_positions=w.keep_positions, **self.kw)
-        self.desc = arr
-        self.count = len(self.windows)
+        self._bind(self.spatial_order and _writes_overlap(self.windows))
         self.graph: Optional[torch.cuda.CUDAGraph] = None
         self._plans = {}
         self.schedule = schedule
 
     # ------------------------------------------------------------------
+    def _bind(self, copies: bool) -> None:
+        """Descriptors over the callers' buffers, or over copies in Morton order."""
+        self._copies = copies
+        if copies:
+            self._sorted = [torch.empty_like(t) for t in self._src]
+            self._bound = [(self._sorted[k], torch.empty_like(w.ftle))
+                           for k, w in zip(self._win_src, self.windows)]
+        else:
+            self._bound = [(w.positions, w.ftle) for w in self.windows]
+        self.desc = (_lib.FtleWindow * self.count)()
+        for i, (w, (pos, ftle)) in enumerate(zip(self.windows, self._bound)):
+            self.desc[i] = window_descriptor(
+                self.series, pos, ftle, h=w.h, num_steps=w.num_steps,
+                map_period=self._map_period[i], t0=w.t0, first_snapshot=w.first_snapshot,
+                keep_positions=w.keep_positions, **self.kw)
+
+    def _rebound(self) -> bool:
+        """Whether a window was given other buffers since the descriptors were built."""
+        return any(w.positions.data_ptr() != (d.positions or 0)
+                   or w.ftle.data_ptr() != (d.ftle or 0)
+                   for w, d in zip(self.windows, self.desc))
+
     def _plan(self, order: int) -> torch.Tensor:
-        if order in self._plans:
-            return self._plans[order]
+        key = (order, self._copies)  # plans that a captured graph may read stay
+        if key in self._plans:
+            return self._plans[key]
         lib = _lib.load()
         nbytes = lib.ftle_windows_plan_bytes(self.desc, self.count)
         if nbytes < 0:
             raise ValueError("invalid batch")
         host = np.zeros(nbytes, dtype=np.uint8)
-        _lib.call("ftle_windows_plan", self.desc, self.count, int(order),
+        orders = (ctypes.c_void_p * self.count)()
+        if self.spatial_order and not self._copies:
+            for i, k in enumerate(self._win_src):
+                orders[i] = self._perm[k].data_ptr()
+        _lib.call("ftle_windows_plan_ordered", self.desc, self.count, int(order), orders,
                   host.ctypes.data_as(ctypes.c_void_p), nbytes)
         dev = torch.from_numpy(host).to(self.windows[0].positions.device)
-        self._plans[order] = dev
+        self._plans[key] = dev
         return dev
 
     def _view(self, t: torch.Tensor) -> torch.Tensor:
@@ -212,19 +250,21 @@ class WindowBatch:
         caller's order."""
         for i, w in enumerate(self.windows):
             k = self._win_src[i]
-            w.ftle.index_copy_(0, self._perm[k], self._win_ftle[i])
+            w.ftle.index_copy_(0, self._perm[k], self._bound[i][1])
             if not w.keep_positions:
                 self._view(w.positions).index_copy_(1, self._perm[k], self._view(self._sorted[k]))
 
     def run(self, schedule: Optional[Schedule] = None, stream=None) -> List[torch.Tensor]:
         sch = schedule or self.schedule
+        if self.spatial_order and not self._copies and self._rebound():
+            self._bind(True)
         plan = self._plan(sch.order)
         with torch.cuda.stream(stream) if stream is not None else contextlib.nullcontext():
-            if self.spatial_order:
+            if self._copies:
                 self._gather()
             _lib.call("ftle_windows_run_mixed", self.desc, self.count, plan.data_ptr(),
                       plan.numel(), int(sch.ctas_per_sm), stream_ptr(stream))
-            if self.spatial_order:
+            if self._copies:
                 self._scatter()
         return [w.ftle for w in self.windows]
 

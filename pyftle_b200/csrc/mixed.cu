@@ -369,6 +369,7 @@ struct WinVar {
   int num_steps, first_snapshot;
   int keep_positions;
   int reserved;
+  const long long *group_order;  // batch: slot -> group, null for the given order
 };
 
 __device__ __forceinline__ WinVar winvar_of(const MixK &m) {
@@ -383,6 +384,7 @@ __device__ __forceinline__ WinVar winvar_of(const MixK &m) {
   v.first_snapshot = m.w.first_snapshot;
   v.keep_positions = m.w.keep_positions;
   v.reserved = 0;
+  v.group_order = nullptr;
   return v;
 }
 
@@ -1366,7 +1368,8 @@ __global__ void __launch_bounds__(kBlock, kMinBlocksPersistent<DIM>)
     const WinVar v = wins[bi.window];
     const long long j_raw = bi.g0 + threadIdx.x;
     const bool active = j_raw < v.N;
-    const long long j = active ? j_raw : v.N - 1;
+    const long long slot = active ? j_raw : v.N - 1;
+    const long long j = v.group_order ? v.group_order[slot] : slot;
     GroupState<DIM> st;
     group_from_positions<DIM>(m, v, j, st);
     group_advect<DIM, MODE, INTEG, STORAGE>(m, v, hd, st, 0, v.num_steps, smem_slots, acc, dsm,
@@ -1664,6 +1667,12 @@ int64_t ftle_windows_plan_bytes(const ftle_window *windows, int32_t count) {
 
 int ftle_windows_plan(const ftle_window *windows, int32_t count, int32_t order, void *host_plan,
                       int64_t plan_bytes) {
+  return ftle_windows_plan_ordered(windows, count, order, nullptr, host_plan, plan_bytes);
+}
+
+int ftle_windows_plan_ordered(const ftle_window *windows, int32_t count, int32_t order,
+                              const int64_t *const *group_orders, void *host_plan,
+                              int64_t plan_bytes) {
   int rc = check_batch(windows, count);
   if (rc) return rc;
   const int64_t ni = batch_items(windows, count);
@@ -1689,6 +1698,8 @@ int ftle_windows_plan(const ftle_window *windows, int32_t count, int32_t order, 
     wins[i].first_snapshot = w.first_snapshot;
     wins[i].keep_positions = (w.flags & FTLE_KEEP_POSITIONS) ? 1 : 0;
     wins[i].reserved = 0;
+    wins[i].group_order =
+        group_orders ? reinterpret_cast<const long long *>(group_orders[i]) : nullptr;
   }
   // order 1: longest windows first (work items of long windows are scheduled before short
   // ones so the tail of the persistent launch is short); order 2: by the start of the
