@@ -390,17 +390,6 @@ __device__ __forceinline__ WinVar winvar_of(const MixK &m) {
 
 __device__ __forceinline__ float lerpf(float a, float b, float t) { return fmaf(t, b - a, a); }
 
-// Wrap a cell index into [0, n): one conditional step covers every index
-// within one period of the grid (the centroid is kept in the primary period).
-__device__ __forceinline__ int wrap_near(int q, int n) {
-  if (q < 0)
-    q += n;
-  else if (q >= n)
-    q -= n;
-  if ((unsigned)q >= (unsigned)n) q = wrap_index(q, n);
-  return q;
-}
-
 // ---------------------------------------------------------------------------
 // packed FP32 (sm_100 FFMA2 / FADD2 / FMUL2): two lanes of one 64-bit register pair
 // per instruction, each lane rounded exactly like the scalar fmaf / add / mul, so
@@ -436,17 +425,40 @@ __device__ __forceinline__ bool cell_values(const MixK &m, const unsigned char *
                                             float alpha, const int *cell, CellVals<DIM> &v) {
   const GridK &g = m.w.g;
   int base = 0, step[DIM];
+  if (g.periodic) {
+    // one conditional step covers every cell within one period of the grid (the centroid is
+    // kept in the primary period); one branch of all axes for those further off, not one each
+    // (turbulence batch 16.2 -> 15.9 ms)
+    int lo[DIM];
+    bool far = false;
 #pragma unroll
-  for (int a = 0; a < DIM; ++a) {
-    int lo = cell[a];
-    step[a] = m.stride[a];
-    if (g.periodic) {
-      lo = wrap_near(lo, g.n[a]);
-      if (lo + 1 == g.n[a]) step[a] = -(g.n[a] - 1) * m.stride[a];
-    } else if (lo < 0 || lo > g.n[a] - 2) {
-      return false;
+    for (int a = 0; a < DIM; ++a) {
+      lo[a] = cell[a];
+      if (lo[a] < 0)
+        lo[a] += g.n[a];
+      else if (lo[a] >= g.n[a])
+        lo[a] -= g.n[a];
+      far = far || (unsigned)lo[a] >= (unsigned)g.n[a];
     }
-    base += lo * m.stride[a];
+    if (far) {
+#pragma unroll
+      for (int a = 0; a < DIM; ++a) lo[a] = wrap_index(lo[a], g.n[a]);
+    }
+#pragma unroll
+    for (int a = 0; a < DIM; ++a) {
+      step[a] = lo[a] + 1 == g.n[a] ? -(g.n[a] - 1) * m.stride[a] : m.stride[a];
+      base += lo[a] * m.stride[a];
+    }
+  } else {
+    bool out = false;
+#pragma unroll
+    for (int a = 0; a < DIM; ++a) out = out || (unsigned)cell[a] >= (unsigned)(g.n[a] - 1);
+    if (out) return false;
+#pragma unroll
+    for (int a = 0; a < DIM; ++a) {
+      step[a] = m.stride[a];
+      base += cell[a] * m.stride[a];
+    }
   }
   const float2 a2 = bc2(alpha);
 #pragma unroll
@@ -598,8 +610,9 @@ __device__ __forceinline__ const unsigned char *record_set(const MixK &m, int s)
 // The lookups of a run of steps, shared by the lanes of a warp (which works on one window):
 // lane kPoints*k + c holds point c (t, t + h/2, t + h; HOLD: the snapshot of the step) of step
 // first + k, so a lookup (~40 instructions, half of them FP64 or conversions, of the ~500 of a
-// 2D warp and stage) runs once per 10 RK4 steps and not per stage: turbulence batch 22.1 ->
-// 20.0 ms, one 512^2 window of 131,072 groups x 80 steps 856 -> 824 us.
+// 2D and ~900 of a 3D warp and stage) runs once per 10 RK4 steps and not per stage: turbulence
+// batch 22.1 -> 20.0 ms, one 512^2 window of 131,072 groups x 80 steps 856 -> 824 us, 3D window
+// of 128^3 groups x 200 steps 68.8 -> 66.9 ms.
 template <int MODE, int INTEG>
 struct StepTimes {
   static constexpr int kPoints = INTEG == FTLE_RK4 && MODE == FTLE_BLEND ? 3 : 1;
@@ -670,8 +683,15 @@ __device__ __forceinline__ void eval_group(const MixK &m, const Header16 &hd,
     const double p = fma(cs[a], m.inv_sp[a], -m.org_sp[a]);
     const double fl = floor(p);
     ok = ok && fabs(fl) < 1.0e9;
-    ci[a] = ok ? (int)fl : 0;
-    fc[a] = ok ? (float)(p - fl) : 0.0f;
+    ci[a] = (int)fl;
+    fc[a] = (float)(p - fl);
+  }
+  if (!__all_sync(0xffffffffu, ok)) {  // non-finite or far centroids: rare, kept off the path
+#pragma unroll
+    for (int a = 0; a < DIM; ++a) {
+      ci[a] = ok ? ci[a] : 0;
+      fc[a] = ok ? fc[a] : 0.0f;
+    }
   }
   float2 fcb[DIM];
 #pragma unroll
@@ -733,7 +753,7 @@ __device__ __forceinline__ void eval_group(const MixK &m, const Header16 &hd,
       for (int i = 0; i < NC; ++i) Ac[i] = c == 0 ? Auv[i].x : (c == 1 ? Auv[i].y : Aw[i]);
       float2 dp = poly_diff_pair<DIM>(Ac, fc[0], g[c], F, dl);
       if constexpr (FX) dp = mul2(bc2(hd.scale[c]), dp);
-      kd[p][c] = make_float2(cin ? dp.x : 0.0f, cin ? dp.y : 0.0f);
+      kd[p][c] = DIM == 2 ? dp : make_float2(cin ? dp.x : 0.0f, cin ? dp.y : 0.0f);
     }
     const int k0 = 2 * p, k1 = 2 * p + 1;
     // 2D stores every neighbour's F without a branch (most warps have an off-cell
@@ -758,6 +778,14 @@ __device__ __forceinline__ void eval_group(const MixK &m, const Header16 &hd,
         for (int a = 0; a < DIM; ++a) slots[(k1 * DIM + a) * kBlock] = F[a].y;
       }
     }
+  }
+  // centroids outside the grid leave zeros; in 3D by selects above (a branch measured 1 % slower)
+  if (DIM == 2 && !__all_sync(0xffffffffu, cin)) {
+#pragma unroll
+    for (int p = 0; p < DIM; ++p)
+#pragma unroll
+      for (int c = 0; c < DIM; ++c)
+        kd[p][c] = make_float2(cin ? kd[p][c].x : 0.0f, cin ? kd[p][c].y : 0.0f);
   }
   if constexpr (DIM == 2) {
     if (!__any_sync(0xffffffffu, off != 0u)) return;
@@ -789,17 +817,19 @@ __device__ __forceinline__ void eval_group(const MixK &m, const Header16 &hd,
         wq.dst[start[k] + __popc(bal[k] & lt)] = k * DIM * kBlock + (int)threadIdx.x;
     }
   } else {
+    // a lane's place by ballots of the bits of its count: one latency, a shuffle scan six
     const int cnt = __popc(off);
-    int incl = cnt;
+    const unsigned lt = (1u << lane) - 1u;
+    int pos = 0;
+    total = 0;
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int y = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += y;
+    for (int i = 0; i < 3; ++i) {
+      const unsigned bal = __ballot_sync(0xffffffffu, (cnt >> i) & 1);
+      pos += __popc(bal & lt) << i;
+      total += __popc(bal) << i;
     }
-    total = __shfl_sync(0xffffffffu, incl, 31);
     if (total == 0) return;  // warp-uniform
     __syncwarp();  // every lane has read its slots of the previous stage
-    int pos = incl - cnt;
 #pragma unroll
     for (int a = 0; a < DIM; ++a) wq.ci[a][lane] = ci[a];
 #pragma unroll
@@ -841,19 +871,11 @@ __device__ __forceinline__ void eval_group(const MixK &m, const Header16 &hd,
   __syncwarp();
 #pragma unroll
   for (int k = 0; k < K; ++k) {
-    if constexpr (DIM == 2) {
 #pragma unroll
-      for (int c = 0; c < DIM; ++c) {
-        const float sv = slots[(k * DIM + c) * kBlock] - uc[c];
-        float &r = (k & 1) ? kd[k >> 1][c].y : kd[k >> 1][c].x;
-        r = (off & (1u << k)) ? sv : r;
-      }
-    } else if (off & (1u << k)) {
-#pragma unroll
-      for (int c = 0; c < DIM; ++c) {
-        float &r = (k & 1) ? kd[k >> 1][c].y : kd[k >> 1][c].x;
-        r = slots[(k * DIM + c) * kBlock] - uc[c];
-      }
+    for (int c = 0; c < DIM; ++c) {
+      const float sv = slots[(k * DIM + c) * kBlock] - uc[c];
+      float &r = (k & 1) ? kd[k >> 1][c].y : kd[k >> 1][c].x;
+      r = (off & (1u << k)) ? sv : r;
     }
   }
 }
@@ -912,12 +934,13 @@ __device__ __forceinline__ void group_from_positions(const MixK &m, const WinVar
 
 // Advect one group through steps [i0, i1) of the window.  The neighbour offsets
 // (dpl) and the RK4 accumulators (accp) live in this thread's shared-memory
-// columns as float2 planes (neighbour pair p = k/2, axis a) at stride kBlock.
+// columns as float2 planes (neighbour pair p = k/2, axis a) at stride kBlock, the
+// counts of removed periods (wraps) in int planes.
 template <int DIM, int MODE, int INTEG, int STORAGE>
 __device__ __forceinline__ void group_advect(const MixK &m, const WinVar &v, const Header16 &hd,
                                              GroupState<DIM> &st, int i0, int i1,
                                              float *smem_slots, float2 *accp, float2 *dpl,
-                                             WarpQueue<DIM> &wq, int lane) {
+                                             int *wraps, WarpQueue<DIM> &wq, int lane) {
   constexpr bool BLEND = MODE == FTLE_BLEND;
   const bool periodic = m.w.g.periodic != 0;
   const double h = v.h;
@@ -930,23 +953,22 @@ __device__ __forceinline__ void group_advect(const MixK &m, const WinVar &v, con
   for (int p = 0; p < DIM; ++p)
 #pragma unroll
     for (int a = 0; a < DIM; ++a) kd[p][a] = make_float2(0.0f, 0.0f);
-  // the offsets live in shared memory during the step loop, which frees 3*K
-  // registers (the kernel then fits 4 blocks per SM)
+  // the offsets and the counts of removed periods live in shared memory during the step loop,
+  // which frees (K + 1) * DIM registers (the kernel then fits 4 blocks per SM)
 #pragma unroll
   for (int p = 0; p < DIM; ++p)
 #pragma unroll
     for (int a = 0; a < DIM; ++a)
       dpl[(p * DIM + a) * kBlock] = make_float2(st.d[2 * p][a], st.d[2 * p + 1][a]);
 
+#pragma unroll
+  for (int a = 0; a < DIM; ++a) wraps[a * kBlock] = st.wraps[a];
   constexpr int NST = INTEG == FTLE_RK4 ? 4 : 1;
-  // in 2D; the 3D kernels have no registers left for the two values (3D batch 2 % slower)
-  constexpr bool kShared = DIM == 2;
   using Times = StepTimes<MODE, INTEG>;
   Times times;
   int k = 0;
   for (int i = i0; i < i1; ++i) {
-    const double t = v.t0 + (double)i * h;
-    if (kShared && k == 0) times.load(m, v, i);
+    if (k == 0) times.load(m, v, i);
 #pragma unroll 1
     for (int s = 0; s < NST; ++s) {
       // RK4 tableau: stage point x + a*k_prev, weight w, time t + tc*h
@@ -955,10 +977,7 @@ __device__ __forceinline__ void group_advect(const MixK &m, const WinVar &v, con
       const float ws = (s == 0 || s == 3) ? 1.0f : 2.0f;
       int set;
       float alpha;
-      if constexpr (kShared)
-        times.at(k, (s + 1) >> 1, set, alpha);
-      else
-        record_time<MODE>(m, v.first_snapshot, i, t + (double)tc * h, set, alpha);
+      times.at(k, (s + 1) >> 1, set, alpha);
       const unsigned char *recs = record_set<DIM>(m, set);
       double cs[DIM];
 #pragma unroll
@@ -1044,7 +1063,7 @@ __device__ __forceinline__ void group_advect(const MixK &m, const WinVar &v, con
           st.kdp[2 * p + 1][a] = kd[p][a].y;
         }
     }
-    if (kShared) k = k + 1 == Times::kSteps ? 0 : k + 1;
+    k = k + 1 == Times::kSteps ? 0 : k + 1;
 #pragma unroll
     for (int a = 0; a < DIM; ++a) {
       kc[a] = 0.0f;  // next step's first stage starts at c
@@ -1052,14 +1071,16 @@ __device__ __forceinline__ void group_advect(const MixK &m, const WinVar &v, con
         const double lo = m.w.g.origin[a], hi = lo + m.period[a];
         if (st.c[a] < lo) {
           st.c[a] += m.period[a];
-          --st.wraps[a];
+          --wraps[a * kBlock];
         } else if (st.c[a] >= hi) {
           st.c[a] -= m.period[a];
-          ++st.wraps[a];
+          ++wraps[a * kBlock];
         }
       }
     }
   }
+#pragma unroll
+  for (int a = 0; a < DIM; ++a) st.wraps[a] = wraps[a * kBlock];
 #pragma unroll
   for (int p = 0; p < DIM; ++p)
 #pragma unroll
@@ -1252,7 +1273,14 @@ __global__ void sort_scatter_kernel(const int *__restrict__ keys, long long N, i
 // the state goes back to `buf` (and its cell key to `keys` when given).
 // Shared memory of a block (dynamic): per-thread columns of the off-cell slots, the
 // RK4 accumulators and the offsets (K*DIM floats each, stride kBlock), then one
-// gather queue per warp.
+// gather queue per warp and the counts of removed periods (DIM ints a thread).
+// What bounds it: latency.  A 3D warp and stage takes ~900 instructions at 0.62 issued per
+// clock with 4 warps a scheduler (128 registers), and the code is larger than what the
+// instruction cache holds for free: sharing a gather pass's items among lanes when the queue is
+// short (3D warps queue 2 to 17 of 192 neighbours a stage) saves instructions but was 4 to 8 %
+// slower wherever both versions of the pass were present.  So registers and code are what is
+// saved: period counts in shared memory, rare cases behind warp-wide branches.  128^3 groups x
+// 200 steps: 70.2 -> 66.9 ms; 2D, 131,072 groups x 80 steps: 826 -> 772 us.
 // Blocks of kBlock threads resident per SM that the register budget is sized for
 // (measured on B200): 4 in 3D; in 2D the persistent batched kernel runs 8 (the
 // turbulence windows keep most neighbours in their cell and gain from latency
@@ -1266,8 +1294,11 @@ constexpr int kMinBlocksPersistent = DIM == 2 ? 8 : 4;
 template <int DIM>
 struct BlockSmem {
   static constexpr int kCol = 2 * DIM * DIM * kBlock;
-  static constexpr size_t kBytes = 3 * kCol * sizeof(float) + (kBlock / 32) * sizeof(WarpQueue<DIM>);
+  static constexpr size_t kBytes = 3 * kCol * sizeof(float) +
+                                   (kBlock / 32) * sizeof(WarpQueue<DIM>) +
+                                   DIM * kBlock * sizeof(int);
   float *slots, *acc, *d;
+  int *wraps;
   WarpQueue<DIM> *queue;
   __device__ explicit BlockSmem(unsigned char *base) {
     float *f = reinterpret_cast<float *>(base);
@@ -1275,6 +1306,7 @@ struct BlockSmem {
     acc = f + kCol;
     d = f + 2 * kCol;
     queue = reinterpret_cast<WarpQueue<DIM> *>(f + 3 * kCol);
+    wraps = reinterpret_cast<int *>(queue + kBlock / 32);
   }
 };
 
@@ -1287,6 +1319,7 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks<DIM>)
   float *smem_slots = sm.slots;
   float2 *acc = reinterpret_cast<float2 *>(sm.acc) + threadIdx.x;
   float2 *dsm = reinterpret_cast<float2 *>(sm.d) + threadIdx.x;
+  int *wraps = sm.wraps + threadIdx.x;
   const int lane = threadIdx.x & 31;
   WarpQueue<DIM> &wq = sm.queue[threadIdx.x >> 5];
   const long long N = m.w.N;
@@ -1307,7 +1340,8 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks<DIM>)
     g = buf.idx[j];
     state_load<DIM>(buf, N, j, st, AB2);
   }
-  group_advect<DIM, MODE, INTEG, STORAGE>(m, v, hd, st, i0, i1, smem_slots, acc, dsm, wq, lane);
+  group_advect<DIM, MODE, INTEG, STORAGE>(m, v, hd, st, i0, i1, smem_slots, acc, dsm, wraps, wq,
+                                          lane);
   if (!active) return;
   if (last) {
     group_finish<DIM>(m, v, g, st);
@@ -1355,6 +1389,7 @@ __global__ void __launch_bounds__(kBlock, kMinBlocksPersistent<DIM>)
   float *smem_slots = sm.slots;
   float2 *acc = reinterpret_cast<float2 *>(sm.acc) + threadIdx.x;
   float2 *dsm = reinterpret_cast<float2 *>(sm.d) + threadIdx.x;
+  int *wraps = sm.wraps + threadIdx.x;
   const int lane = threadIdx.x & 31;
   WarpQueue<DIM> &wq = sm.queue[threadIdx.x >> 5];
   const Header16 hd = *reinterpret_cast<const Header16 *>(m.w.snaps);
@@ -1373,12 +1408,12 @@ __global__ void __launch_bounds__(kBlock, kMinBlocksPersistent<DIM>)
     GroupState<DIM> st;
     group_from_positions<DIM>(m, v, j, st);
     group_advect<DIM, MODE, INTEG, STORAGE>(m, v, hd, st, 0, v.num_steps, smem_slots, acc, dsm,
-                                            wq, lane);
+                                            wraps, wq, lane);
     if (active) group_finish<DIM>(m, v, j, st);
   }
 }
 
-// Allow the kernel's dynamic shared memory (31.5 KB for a 3D block, 15 KB in 2D, under
+// Allow the kernel's dynamic shared memory (33 KB for a 3D block, 16 KB in 2D, under
 // the 48 KB default today; set anyway so a larger layout needs no other change);
 // called once per kernel instance.
 template <typename Kernel>
