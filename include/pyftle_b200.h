@@ -172,6 +172,18 @@ int ftle_pack_snapshots(int32_t dim, int64_t nodes, int32_t num_snapshots,
  * pyFTLE's positions; FTLE within 1e-10 relative. */
 int ftle_window_run_f64(const ftle_window *w, void *stream);
 
+/* Plain FP64 sample of a window of any storage: every stride-th group (0, stride, ...) of
+ * `seeds` ((2*dim*num_groups, dim), only read) is advected over `source`, the window's
+ * (num_snapshots, dim, nodes) float64 snapshots, and its FTLE written to `sample`
+ * (ceil(num_groups / stride) doubles): the bits that ftle_window_run_f64 gives those groups
+ * over the packed series.  The descriptor's snapshots, positions and ftle are not touched. */
+int ftle_window_sample_f64(const ftle_window *w, const double *source, const double *seeds,
+                           int64_t stride, double *sample, void *stream);
+/* Sums of squares of field[i*stride] - sample[i] and of sample[i]: `blocks` pairs of doubles
+ * (16-byte aligned), whose sums over the pairs are the squared norms. */
+int ftle_sample_norms(const double *field, const double *sample, int64_t num_groups,
+                      int64_t stride, double *sums, int32_t blocks, void *stream);
+
 /* Mixed-precision window (storage FTLE_F16, FTLE_BF16, FTLE_FX15 or FTLE_FX16): FP32 advection of
  * each group as an FP64 centroid plus FP32 neighbour offsets (split
  * representation), FP64 Jacobian -> Cauchy-Green -> lambda_max.  Writes

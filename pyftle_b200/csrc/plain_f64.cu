@@ -249,6 +249,38 @@ __device__ __forceinline__ void velocity_packed(const GridK &g, const double *__
   for (int comp = 0; comp < DIM; ++comp) u[comp] = interp_corners<DIM>(last.v[comp], c.f);
 }
 
+// The same velocity from the snapshots as the caller has them, (S, dim, nodes): the successor's
+// corners are read and blended in the records' order, so the bits are those of packed records.
+template <int DIM, bool BLEND>
+__device__ __forceinline__ void velocity_source(const WinK &w, int s, double alpha,
+                                                const double *x, double *u) {
+  const GridK &g = w.g;
+  const long long set = g.nodes * DIM;
+  Cell64<DIM> c;
+  if (!locate64<DIM, 8>(g, static_cast<const double *>(w.snaps) + s * set, x, c)) {
+#pragma unroll
+    for (int a = 0; a < DIM; ++a) u[a] = 0.0;
+    return;
+  }
+  const int next = s + 1 < w.num_snaps ? s + 1 : (w.periodic_time ? 0 : w.num_snaps - 1);
+  const long long to_next = (next - s) * set * 8;
+  const double oma = 1.0 - alpha;
+  const char *r[1 << DIM];
+  corners<DIM>(c, r);
+#pragma unroll
+  for (int comp = 0; comp < DIM; ++comp) {
+    double v[1 << DIM];
+#pragma unroll
+    for (int q = 0; q < (1 << DIM); ++q) {
+      const char *p = r[q] + comp * g.nodes * 8;
+      v[q] = __ldg(reinterpret_cast<const double *>(p));
+      if constexpr (BLEND)
+        v[q] = v[q] * oma + __ldg(reinterpret_cast<const double *>(p + to_next)) * alpha;
+    }
+    u[comp] = interp_corners<DIM>(v, c.f);
+  }
+}
+
 // ---------------------------------------------------------------------------
 // time lookup (BLEND)
 // ---------------------------------------------------------------------------
@@ -296,7 +328,7 @@ struct StepTimes {
 };
 
 // Velocity at point c of the k-th step of `times` (step number `step`).
-template <int DIM, bool TRY, int MODE, int INTEG>
+template <int DIM, bool TRY, bool SOURCE, int MODE, int INTEG>
 __device__ __forceinline__ void field(const WinK &w, const StepTimes<MODE, INTEG> &times, int k,
                                       int step, int c, const double *x, double *u,
                                       Corners64<DIM> &last) {
@@ -305,18 +337,25 @@ __device__ __forceinline__ void field(const WinK &w, const StepTimes<MODE, INTEG
   if constexpr (MODE == FTLE_HOLD) {
     int s = w.first_snapshot + step;
     if (w.periodic_time) s %= w.num_snaps;
-    velocity_packed<DIM, false, TRY>(w.g, recs + s * rec_set, 0.0, x, u, last);
+    if constexpr (SOURCE)
+      velocity_source<DIM, false>(w, s, 0.0, x, u);
+    else
+      velocity_packed<DIM, false, TRY>(w.g, recs + s * rec_set, 0.0, x, u, last);
   } else {
     const int lane = k * times.kPoints + c;
     const int s = __shfl_sync(0xffffffffu, times.s, lane);
     const double alpha = __shfl_sync(0xffffffffu, times.alpha, lane);
-    velocity_packed<DIM, true, TRY>(w.g, recs + s * rec_set, alpha, x, u, last);
+    if constexpr (SOURCE)
+      velocity_source<DIM, true>(w, s, alpha, x, u);
+    else
+      velocity_packed<DIM, true, TRY>(w.g, recs + s * rec_set, alpha, x, u, last);
   }
 }
 
 // One particle through the whole window (integrate.py restated step by step).  All lanes of
-// a warp take part (the time lookups are shared).
-template <int DIM, int MODE, int INTEG>
+// a warp take part (the time lookups are shared).  SOURCE: w.snaps are the snapshots as the
+// caller has them, not records.
+template <int DIM, int MODE, int INTEG, bool SOURCE = false>
 __device__ __forceinline__ void advect(const WinK &w, double *x) {
   const double h = w.h;
   double vprev[DIM];
@@ -329,12 +368,12 @@ __device__ __forceinline__ void advect(const WinK &w, double *x) {
       const int i = first + k;
       if constexpr (INTEG == FTLE_EULER) {
         double v[DIM];
-        field<DIM, false>(w, times, k, i, 0, x, v, last);
+        field<DIM, false, SOURCE>(w, times, k, i, 0, x, v, last);
 #pragma unroll
         for (int a = 0; a < DIM; ++a) x[a] = x[a] + h * v[a];
       } else if constexpr (INTEG == FTLE_AB2) {
         double v[DIM];
-        field<DIM, false>(w, times, k, i, 0, x, v, last);
+        field<DIM, false, SOURCE>(w, times, k, i, 0, x, v, last);
         if (i == 0) {
 #pragma unroll
           for (int a = 0; a < DIM; ++a) x[a] = x[a] + h * v[a];
@@ -350,25 +389,25 @@ __device__ __forceinline__ void advect(const WinK &w, double *x) {
         // loads would be saved, the test cost more than they did (2D 4 %, 3D 5 % slower)
         constexpr bool kTry = MODE == FTLE_BLEND;
         double kv[DIM], acc[DIM], tmp[DIM];
-        field<DIM, kTry>(w, times, k, i, 0, x, kv, last);
+        field<DIM, kTry, SOURCE>(w, times, k, i, 0, x, kv, last);
 #pragma unroll
         for (int a = 0; a < DIM; ++a) {
           acc[a] = kv[a];
           tmp[a] = x[a] + hh * kv[a];
         }
-        field<DIM, false>(w, times, k, i, 1, tmp, kv, last);
+        field<DIM, false, SOURCE>(w, times, k, i, 1, tmp, kv, last);
 #pragma unroll
         for (int a = 0; a < DIM; ++a) {
           acc[a] = acc[a] + 2.0 * kv[a];
           tmp[a] = x[a] + hh * kv[a];
         }
-        field<DIM, kTry>(w, times, k, i, 1, tmp, kv, last);
+        field<DIM, kTry, SOURCE>(w, times, k, i, 1, tmp, kv, last);
 #pragma unroll
         for (int a = 0; a < DIM; ++a) {
           acc[a] = acc[a] + 2.0 * kv[a];
           tmp[a] = x[a] + h * kv[a];
         }
-        field<DIM, false>(w, times, k, i, 2, tmp, kv, last);
+        field<DIM, false, SOURCE>(w, times, k, i, 2, tmp, kv, last);
         const double h6 = h / 6.0;
 #pragma unroll
         for (int a = 0; a < DIM; ++a) x[a] = x[a] + h6 * (acc[a] + kv[a]);
@@ -498,6 +537,76 @@ __global__ void __launch_bounds__(2 * DIM * kGroups<DIM, MODE>, kBlocksPerSM<DIM
       }
     }
   }
+}
+
+// FTLE of every stride-th group of a window, straight from the snapshots as the caller has
+// them: the sample that judges a 16-bit window.  One thread per particle, one warp (3D: three)
+// per block, so that a sample spreads over the SMs; it is one FP64 chain long whatever its size
+// (1,311 groups of a 512^2 window, 80 steps: 0.17 ms on 164 of the chip's 592 schedulers), which
+// is why the caller runs it beside the window itself.  Records of the whole series for a sample
+// of 1 % took 76 us to write and twice the series' memory.
+template <int DIM>
+constexpr int kSampleGroups = DIM == 2 ? 8 : 16;
+
+template <int DIM, int MODE, int INTEG>
+__global__ void __launch_bounds__(2 * DIM * kSampleGroups<DIM>)
+    sample_f64_kernel(const WinK w, long long stride, long long samples) {
+  constexpr int G = kSampleGroups<DIM>;
+  constexpr int K = 2 * DIM;
+  __shared__ double sx[K][G][DIM];
+  __shared__ double sx0[K][G][DIM];
+  const int role = threadIdx.x % K, gl = threadIdx.x / K;
+  const long long i = (long long)blockIdx.x * G + gl;
+  // threads past the last group repeat it: a warp's lanes share time lookups
+  const long long row = (long long)role * w.N + min(i, samples - 1) * stride;
+  double x[DIM];
+#pragma unroll
+  for (int a = 0; a < DIM; ++a) {
+    x[a] = w.positions[row * DIM + a];
+    sx0[role][gl][a] = x[a];
+  }
+  advect<DIM, MODE, INTEG, true>(w, x);
+#pragma unroll
+  for (int a = 0; a < DIM; ++a) sx[role][gl][a] = x[a];
+  __syncthreads();
+  const long long out = (long long)blockIdx.x * G + threadIdx.x;
+  if (threadIdx.x < G && out < samples) {
+    double P[K][DIM], id[DIM];
+#pragma unroll
+    for (int r = 0; r < K; ++r)
+#pragma unroll
+      for (int a = 0; a < DIM; ++a) P[r][a] = sx[r][threadIdx.x][a];
+#pragma unroll
+    for (int j = 0; j < DIM; ++j)
+      id[j] = sx0[plus_role(j)][threadIdx.x][j] - sx0[minus_role(j)][threadIdx.x][j];
+    w.ftle[out] = group_ftle<DIM>(P, id, w.map_period);
+  }
+}
+
+// Sums of squares of (field[i * stride] - sample[i]) and sample[i], one pair per block.
+constexpr int kNormThreads = 256;
+
+__global__ void __launch_bounds__(kNormThreads)
+    sample_norms_kernel(const double *__restrict__ field, const double *__restrict__ sample,
+                        long long stride, long long samples, double2 *sums) {
+  double2 s = make_double2(0.0, 0.0);
+  for (long long i = blockIdx.x * (long long)kNormThreads + threadIdx.x; i < samples;
+       i += (long long)gridDim.x * kNormThreads) {
+    const double r = sample[i], d = field[i * stride] - r;
+    s.x += d * d;
+    s.y += r * r;
+  }
+  __shared__ double2 part[kNormThreads];
+  part[threadIdx.x] = s;
+  __syncthreads();
+  for (int half = kNormThreads / 2; half > 0; half >>= 1) {
+    if (threadIdx.x < half) {
+      part[threadIdx.x].x += part[threadIdx.x + half].x;
+      part[threadIdx.x].y += part[threadIdx.x + half].y;
+    }
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) sums[blockIdx.x] = part[0];
 }
 
 // ---------------------------------------------------------------------------
@@ -1057,6 +1166,24 @@ static void launch_window(const WinK &w, cudaStream_t st) {
   window_f64_kernel<DIM, MODE, INTEG><<<(unsigned)blocks, 2 * DIM * G, 0, st>>>(w);
 }
 
+template <int DIM, int MODE, int INTEG>
+static void launch_sample(const WinK &w, long long stride, long long samples, cudaStream_t st) {
+  constexpr int G = kSampleGroups<DIM>;
+  sample_f64_kernel<DIM, MODE, INTEG>
+      <<<(unsigned)((samples + G - 1) / G), 2 * DIM * G, 0, st>>>(w, stride, samples);
+}
+
+template <int DIM, int MODE>
+static void launch_sample_i(const WinK &w, int integ, long long stride, long long samples,
+                            cudaStream_t st) {
+  if (integ == FTLE_EULER)
+    launch_sample<DIM, MODE, FTLE_EULER>(w, stride, samples, st);
+  else if (integ == FTLE_AB2)
+    launch_sample<DIM, MODE, FTLE_AB2>(w, stride, samples, st);
+  else
+    launch_sample<DIM, MODE, FTLE_RK4>(w, stride, samples, st);
+}
+
 template <int DIM, int MODE>
 static void launch_window_i(const WinK &w, int integ, cudaStream_t st) {
   if (integ == FTLE_EULER)
@@ -1093,6 +1220,48 @@ int ftle_window_run_f64(const ftle_window *w, void *stream) {
       launch_window_i<3, FTLE_BLEND>(k, w->integrator, st);
   }
   return check_launch("window_f64_kernel");
+}
+
+int ftle_window_sample_f64(const ftle_window *w, const double *source, const double *seeds,
+                           int64_t stride, double *sample, void *stream) {
+  WinK k;
+  int rc = window_to_kernel(w, &k);
+  if (rc) return rc;
+  if (stride < 1) return fail_invalid("stride must be >= 1");
+  const int64_t samples = (k.N + stride - 1) / stride;
+  if (samples == 0) return FTLE_OK;
+  if (!source || !seeds || !sample) return fail_invalid("null pointer");
+  if (!(k.map_period > 0.0) && !(k.map_period < 0.0))
+    return fail_invalid("map_period must be non-zero");
+  k.snaps = source;
+  k.positions = const_cast<double *>(seeds);
+  k.ftle = sample;
+  cudaStream_t st = as_stream(stream);
+  if (w->grid.dim == 2) {
+    if (w->time_mode == FTLE_HOLD)
+      launch_sample_i<2, FTLE_HOLD>(k, w->integrator, stride, samples, st);
+    else
+      launch_sample_i<2, FTLE_BLEND>(k, w->integrator, stride, samples, st);
+  } else {
+    if (w->time_mode == FTLE_HOLD)
+      launch_sample_i<3, FTLE_HOLD>(k, w->integrator, stride, samples, st);
+    else
+      launch_sample_i<3, FTLE_BLEND>(k, w->integrator, stride, samples, st);
+  }
+  return check_launch("sample_f64_kernel");
+}
+
+int ftle_sample_norms(const double *field, const double *sample, int64_t num_groups,
+                      int64_t stride, double *sums, int32_t blocks, void *stream) {
+  if (stride < 1) return fail_invalid("stride must be >= 1");
+  if (blocks < 1 || num_groups < 0) return fail_invalid("sizes must be positive");
+  if (!sums || (num_groups > 0 && (!field || !sample))) return fail_invalid("null pointer");
+  if (reinterpret_cast<uintptr_t>(sums) % 16 != 0)
+    return fail_invalid("sums must be 16-byte aligned");
+  sample_norms_kernel<<<(unsigned)blocks, kNormThreads, 0, as_stream(stream)>>>(
+      field, sample, stride, (num_groups + stride - 1) / stride,
+      reinterpret_cast<double2 *>(sums));
+  return check_launch("sample_norms_kernel");
 }
 
 int ftle_interp2d_vec_inplace(const double *v, int32_t nx, int32_t ny, const double *points,

@@ -35,7 +35,8 @@ from pyftle_b200.data_source import BatchSource
 from pyftle_b200.ftle import compute_ftle_from_positions
 from pyftle_b200.integrate import Integrator
 from pyftle_b200.interpolate import HighPerfInterpolator
-from pyftle_b200.window import EngineOptions, SnapshotSeries, run_window
+from pyftle_b200.window import (EngineOptions, SnapshotSeries, run_window, sample_error,
+                                sample_window_f64)
 
 
 class FTLESolver:
@@ -68,12 +69,10 @@ class FTLESolver:
                        num_steps=spec.num_steps, map_period=spec.map_period, t0=spec.t0,
                        first_snapshot=spec.first_snapshot, snapshot_t0=spec.snapshot_t0,
                        snapshot_dt=spec.snapshot_dt)
-            seeds = self.particles.positions.clone() if judge else None
-            ftle = run_window(self.series, self.particles.positions,
-                              chunk_steps=self.options.chunk_steps,
-                              sort_every=self.options.sort_every, **win)
-            if judge:
-                ftle = self._judge(ftle, seeds, spec, win)
+            run = lambda: run_window(self.series, self.particles.positions,  # noqa: E731
+                                     chunk_steps=self.options.chunk_steps,
+                                     sort_every=self.options.sort_every, **win)
+            ftle = self._judged(run, spec, win) if judge else run()
             if self.progress_queue:
                 for i in range(spec.num_steps):
                     self.progress_queue.put((ident, i))
@@ -108,31 +107,39 @@ class FTLESolver:
             return None
         return field
 
-    def _judge(self, ftle: torch.Tensor, seeds: torch.Tensor, spec, win) -> torch.Tensor:
-        """FP64 judge of a mixed-precision window: the plain FP64 kernel advects every
-        ``judge_stride``-th group of the window's seeds; if the sampled FTLE's relative
-        L2 error exceeds ``judge_tol`` (or is not finite), the whole window is re-advected
-        by the plain FP64 kernel (FTLE and final positions become the FP64 ones).  The
-        outcome is left in ``self.judge``."""
+    def _judged(self, run, spec, win) -> torch.Tensor:
+        """``run()`` (a mixed-precision window) under the FP64 judge: every
+        ``judge_stride``-th group of the window's seeds is advected in plain FP64; if the
+        sampled FTLE's relative L2 error exceeds ``judge_tol`` (or is not finite), the whole
+        window is re-advected by the plain FP64 kernel (FTLE and final positions become the
+        FP64 ones).  The outcome is left in ``self.judge``.
+
+        The sample is one long FP64 chain on a few warps, so it runs beside the window on a
+        stream of its own, which joins the caller's stream before anything else happens.
+        Every tensor belongs to the caller's stream."""
         opts = self.options
         stride = max(1, int(opts.judge_stride))
-        K = 2 * spec.grid.dim
-        n = seeds.shape[0] // K
-        sel = torch.arange(0, n, stride, device=seeds.device)
-        sub = seeds.view(K, n, spec.grid.dim)[:, sel, :].reshape(-1, spec.grid.dim).contiguous()
-        series64 = SnapshotSeries(spec.grid, self.series.source, precision="fp64",
-                                  periodic_time=spec.periodic_time)
-        self.series.source = None
-        f64 = run_window(series64, sub, **win)
-        ref = torch.linalg.vector_norm(f64)
-        diff = torch.linalg.vector_norm(ftle[sel] - f64)
-        err = float(diff / ref) if float(ref) > 0 else float(diff)
+        positions = self.particles.positions
+        seeds = positions.clone()
+        n = seeds.shape[0] // (2 * spec.grid.dim)
+        sample = torch.empty(-(-n // stride), dtype=torch.float64, device=seeds.device)
+        current, side = torch.cuda.current_stream(), torch.cuda.Stream()
+        side.wait_stream(current)
+        try:
+            sample_window_f64(self.series, seeds, stride, sample, side, **win)
+            ftle = run()
+        finally:
+            current.wait_stream(side)
+        err = sample_error(ftle, sample, stride)
         redo = not err <= opts.judge_tol
         if redo:
+            series64 = SnapshotSeries(spec.grid, self.series.source, precision="fp64",
+                                      periodic_time=spec.periodic_time)
             ftle = run_window(series64, seeds, **win)
-            self.particles.positions.copy_(seeds)
+            positions.copy_(seeds)
+        self.series.source = None
         self.judge = {"error": err, "tol": float(opts.judge_tol), "readvected": redo,
-                      "sample_groups": int(sel.numel())}
+                      "sample_groups": sample.numel()}
         return ftle
 
     def _compute_ftle(self) -> np.ndarray:

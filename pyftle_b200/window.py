@@ -18,6 +18,7 @@ Time modes:
 
 from __future__ import annotations
 
+import math
 from dataclasses import dataclass
 from typing import Optional
 
@@ -117,6 +118,18 @@ def window_descriptor(series: SnapshotSeries, positions: torch.Tensor, ftle: Opt
     return w
 
 
+def _window_defaults(integrator, time_mode, h, num_steps, map_period, snapshot_dt):
+    if time_mode not in _lib.TIME_MODES:
+        raise ValueError(f"time_mode must be one of {list(_lib.TIME_MODES)}")
+    if integrator.lower() not in _lib.INTEGRATOR_CODES:
+        raise ValueError(f"Invalid integrator name '{integrator}'.")
+    if map_period is None:
+        map_period = (num_steps - 1) * abs(h) if time_mode == "hold" else num_steps * abs(h)
+    if snapshot_dt is None:
+        snapshot_dt = h if time_mode == "hold" else 1.0
+    return map_period, snapshot_dt
+
+
 def run_window(series: SnapshotSeries, positions: torch.Tensor, *, integrator: str = "rk4",
                time_mode: str = "hold", h: float, num_steps: int,
                map_period: Optional[float] = None, t0: float = 0.0, first_snapshot: int = 0,
@@ -132,14 +145,8 @@ def run_window(series: SnapshotSeries, positions: torch.Tensor, *, integrator: s
     ``workspace`` is given) and a cell sort of the groups every ``sort_every``
     chunks.
     """
-    if time_mode not in _lib.TIME_MODES:
-        raise ValueError(f"time_mode must be one of {list(_lib.TIME_MODES)}")
-    if integrator.lower() not in _lib.INTEGRATOR_CODES:
-        raise ValueError(f"Invalid integrator name '{integrator}'.")
-    if map_period is None:
-        map_period = (num_steps - 1) * abs(h) if time_mode == "hold" else num_steps * abs(h)
-    if snapshot_dt is None:
-        snapshot_dt = h if time_mode == "hold" else 1.0
+    map_period, snapshot_dt = _window_defaults(integrator, time_mode, h, num_steps, map_period,
+                                               snapshot_dt)
     K = 2 * series.grid.dim
     n = positions.shape[0] // K
     ftle = None
@@ -161,3 +168,31 @@ def run_window(series: SnapshotSeries, positions: torch.Tensor, *, integrator: s
         _lib.call("ftle_window_run_mixed_chunked", w, workspace.data_ptr(), workspace.numel(),
                   int(chunk_steps), int(sort_every), stream_ptr(stream))
     return ftle
+
+
+def sample_window_f64(series: SnapshotSeries, seeds: torch.Tensor, stride: int, out: torch.Tensor,
+                      stream: torch.cuda.Stream, *, integrator: str, time_mode: str, h: float,
+                      num_steps: int, map_period: Optional[float], t0: float,
+                      first_snapshot: int, snapshot_t0: float,
+                      snapshot_dt: Optional[float]) -> None:
+    """Plain FP64 FTLE of every ``stride``-th group of ``seeds`` into ``out``, on ``stream``,
+    from ``series.source`` (the series keeps it): no FP64 records are packed.  The caller
+    orders ``stream`` after the tensors' own stream, and that one after ``stream``."""
+    map_period, snapshot_dt = _window_defaults(integrator, time_mode, h, num_steps, map_period,
+                                               snapshot_dt)
+    w = window_descriptor(series, seeds, None, integrator=integrator, time_mode=time_mode, h=h,
+                          num_steps=num_steps, map_period=map_period, t0=t0,
+                          first_snapshot=first_snapshot, snapshot_t0=snapshot_t0,
+                          snapshot_dt=snapshot_dt, keep_positions=True)
+    _lib.call("ftle_window_sample_f64", w, ptr(series.source), ptr(seeds), int(stride), ptr(out),
+              stream_ptr(stream))
+
+
+def sample_error(field: torch.Tensor, sample: torch.Tensor, stride: int) -> float:
+    """||field[::stride] - sample|| / ||sample|| (the absolute norm where the sample is zero)."""
+    blocks = max(1, min(148, -(-sample.numel() // 1024)))
+    sums = torch.empty((blocks, 2), dtype=torch.float64, device=field.device)
+    _lib.call("ftle_sample_norms", ptr(field), ptr(sample), field.numel(), int(stride), ptr(sums),
+              blocks, stream_ptr())
+    diff, ref = sums.cpu().numpy().sum(axis=0)
+    return math.sqrt(diff) / math.sqrt(ref) if ref > 0 else math.sqrt(diff)
