@@ -36,3 +36,28 @@ def test_odd_neighbours_leave_a_group_alone(dim, periodic, chunk):
     np.testing.assert_array_equal(out[0][0], out[1][0])
     np.testing.assert_array_equal(out[0][1], out[1][1])
     assert np.isfinite(out[0][0]).all()
+
+
+@pytest.mark.parametrize("dim", [2, 3])
+@pytest.mark.parametrize("integ", ["euler", "ab2", "rk4"])
+@pytest.mark.parametrize("groups", [1, 127, 129, 4000])
+@pytest.mark.parametrize("sort_every", [0, 1, 2])
+def test_chunks_keep_the_bits_of_one_launch(dim, integ, groups, sort_every):
+    """Groups travel from chunk to chunk through the sort's order: records, tags and AB2
+    history arrive with their group, whichever chunks are sorted."""
+    rng = np.random.default_rng(4)
+    n = (19, 16, 17)[:dim]
+    grid = GridSpec(n, (0.0,) * dim, tuple(1.0 / k for k in n), True)
+    series = SnapshotSeries(grid, rng.uniform(-3, 3, (4, dim, int(np.prod(n)))),
+                            precision="fx15")
+    seeds = (flows.seeds_2d if dim == 2 else flows.seeds_3d)(
+        rng.uniform(0, 1, (groups, dim)), 5e-3)
+    out = []
+    for chunk in (None, 3):
+        pos = torch.as_tensor(seeds, device="cuda")
+        f = run_window(series, pos, integrator=integ, time_mode="blend", h=0.02, num_steps=14,
+                       snapshot_dt=0.1, chunk_steps=chunk, sort_every=sort_every)
+        torch.cuda.synchronize()
+        out.append((f.cpu().numpy(), pos.cpu().numpy()))
+    np.testing.assert_array_equal(out[0][0], out[1][0])
+    np.testing.assert_array_equal(out[0][1], out[1][1])
