@@ -462,13 +462,13 @@ def run_ours(args):
         assert np.isfinite(field).all()
         del snaps_pin, pos_pin
 
-    # our kernels per window: one launch per chunk, plus 3 sort kernels per sorted boundary
+    # our kernels per window: one launch per chunk, plus 2 sort kernels per sorted boundary
     if chunk is None:
         launches_per_window = 1
     else:
         nch = -(-w["num_steps"] // chunk)
         nsort = sum(1 for ci in range(nch - 1) if args.sort_every > 0 and (ci + 1) % args.sort_every == 0)
-        launches_per_window = nch + 3 * nsort
+        launches_per_window = nch + 2 * nsort
 
     # --- roofline of the dominant kernel --------------------------------------
     # The window kernel gathers 16-byte snapshot records from an L1/L2-resident working
@@ -1284,11 +1284,10 @@ def run_surrogate3d(args):
         "ftle_rel_err_l2_judged_vs_rk4": {"max": max(judged_err), "mean": float(np.mean(judged_err))},
         "surrogate_and_judge_ms_per_field": eval_ms, "rk4_ms_per_field": rk_ms,
         "tolerance_sweep": sweep_out,
-        # per window: per 2^20-seed chunk the feature kernel, 4 primal + 1 output GEMM,
-        # 3 tangent passes of 5 GEMMs and the FTLE kernel (22); the judge's RK4 window
-        # (2 chunk launches + one 3-kernel cell sort); the same again when any region
+        # per window: the weights' packing and the field kernel; the judge's RK4 window
+        # (2 chunk launches + one 2-kernel cell sort); the same again when any region
         # is re-advected
-        "gpu_launches": W * (22 * (-(-m ** 3 // (1 << 20))) + 5) + 5 * readv_windows,
+        "gpu_launches": W * (2 + 4) + 4 * readv_windows,
     }
     print(json.dumps(line), flush=True)
     return 0
