@@ -649,6 +649,23 @@ __device__ __forceinline__ double lmax2(double F00, double F01, double F10, doub
 }
 
 
+// A neighbour pair's DIM float2 values in a block's shared-memory array: axes 0 and 1 as one
+// 16-byte column, axis 2 in an 8-byte column after it.
+template <int DIM>
+__device__ __forceinline__ void pair_get(const float2 *base, int p, float2 *v) {
+  const float2 *b = base + p * DIM * kBlock;
+  const float4 f = reinterpret_cast<const float4 *>(b)[threadIdx.x];
+  v[0] = make_float2(f.x, f.y);
+  v[1] = make_float2(f.z, f.w);
+  if constexpr (DIM == 3) v[2] = b[2 * kBlock + threadIdx.x];
+}
+template <int DIM>
+__device__ __forceinline__ void pair_put(float2 *base, int p, const float2 *v) {
+  float2 *b = base + p * DIM * kBlock;
+  reinterpret_cast<float4 *>(b)[threadIdx.x] = make_float4(v[0].x, v[0].y, v[1].x, v[1].y);
+  if constexpr (DIM == 3) b[2 * kBlock + threadIdx.x] = v[2];
+}
+
 // Off-cell neighbour work items of one warp.  An item is the slot index of the
 // owning thread's neighbour (its in-cell coordinates F relative to the owner's
 // centroid cell wait in that slot); the owners' centroid cells sit beside it.
@@ -664,7 +681,7 @@ struct WarpQueue {
 // k = 2p, 2p+1 (lanes .x, .y).  Neighbours inside the centroid's cell use the
 // cell polynomial; the others are queued per warp and gathered 32 at a time, so
 // no lane idles in a divergent loop.  `dpl`: this thread's offsets in shared
-// memory, float2 planes (neighbour pair p, axis a) at stride kBlock.
+// memory (pair_get).
 template <int DIM, int STORAGE, bool BLEND>
 __device__ __forceinline__ void eval_group(const MixK &m, const Header16 &hd,
                                            const unsigned char *__restrict__ recs, float alpha,
@@ -736,16 +753,20 @@ __device__ __forceinline__ void eval_group(const MixK &m, const Header16 &hd,
   const float2 as2 = bc2(as);
 #pragma unroll
   for (int p = 0; p < DIM; ++p) {
-    float2 dl[DIM], F[DIM];
-    bool same0 = true, same1 = true;
+    float2 dl[DIM], F[DIM], d0[DIM];
+    pair_get<DIM>(dpl, p, d0);
+    // a coordinate is in [0, 1) exactly when its bits are below 1.0f's: -0 cannot arise (a cell
+    // fraction is +0 or more, and a sum that cancels is +0), negatives and NaN lie above
+    unsigned most0 = 0u, most1 = 0u;
 #pragma unroll
     for (int a = 0; a < DIM; ++a) {
       // explicit roundings: the cell test and the polynomial use the same F and dl
-      dl[a] = mul2(fma2(as2, kd[p][a], dpl[(p * DIM + a) * kBlock]), bc2(m.inv_spf[a]));
+      dl[a] = mul2(fma2(as2, kd[p][a], d0[a]), bc2(m.inv_spf[a]));
       F[a] = add2(fcb[a], dl[a]);
-      same0 = same0 && F[a].x >= 0.0f && F[a].x < 1.0f;
-      same1 = same1 && F[a].y >= 0.0f && F[a].y < 1.0f;
+      most0 = max(most0, __float_as_uint(F[a].x));
+      most1 = max(most1, __float_as_uint(F[a].y));
     }
+    const bool same0 = most0 < 0x3f800000u, same1 = most1 < 0x3f800000u;
 #pragma unroll
     for (int c = 0; c < DIM; ++c) {
       float Ac[NC];
@@ -934,8 +955,8 @@ __device__ __forceinline__ void group_from_positions(const MixK &m, const WinVar
 
 // Advect one group through steps [i0, i1) of the window.  The neighbour offsets
 // (dpl) and the RK4 accumulators (accp) live in this thread's shared-memory
-// columns as float2 planes (neighbour pair p = k/2, axis a) at stride kBlock, the
-// counts of removed periods (wraps) in int planes.
+// columns by neighbour pair p = k/2 (pair_get: 16 bytes an access, 6 instead of 9 a
+// stage in 3D), the counts of removed periods (wraps) in int planes.
 template <int DIM, int MODE, int INTEG, int STORAGE>
 __device__ __forceinline__ void group_advect(const MixK &m, const WinVar &v, const Header16 &hd,
                                              GroupState<DIM> &st, int i0, int i1,
@@ -956,10 +977,12 @@ __device__ __forceinline__ void group_advect(const MixK &m, const WinVar &v, con
   // the offsets and the counts of removed periods live in shared memory during the step loop,
   // which frees (K + 1) * DIM registers (the kernel then fits 4 blocks per SM)
 #pragma unroll
-  for (int p = 0; p < DIM; ++p)
+  for (int p = 0; p < DIM; ++p) {
+    float2 d0[DIM];
 #pragma unroll
-    for (int a = 0; a < DIM; ++a)
-      dpl[(p * DIM + a) * kBlock] = make_float2(st.d[2 * p][a], st.d[2 * p + 1][a]);
+    for (int a = 0; a < DIM; ++a) d0[a] = make_float2(st.d[2 * p][a], st.d[2 * p + 1][a]);
+    pair_put<DIM>(dpl, p, d0);
+  }
 
 #pragma unroll
   for (int a = 0; a < DIM; ++a) wraps[a * kBlock] = st.wraps[a];
@@ -996,12 +1019,13 @@ __device__ __forceinline__ void group_advect(const MixK &m, const WinVar &v, con
         if (s < 3) {
           const float2 ws2 = bc2(ws);
 #pragma unroll
-          for (int p = 0; p < DIM; ++p)
+          for (int p = 0; p < DIM; ++p) {
+            float2 r[DIM];
+            if (s > 0) pair_get<DIM>(accp, p, r);
 #pragma unroll
-            for (int a = 0; a < DIM; ++a) {
-              float2 &r = accp[(p * DIM + a) * kBlock];
-              r = s == 0 ? kd[p][a] : fma2(ws2, kd[p][a], r);
-            }
+            for (int a = 0; a < DIM; ++a) r[a] = s == 0 ? kd[p][a] : fma2(ws2, kd[p][a], r[a]);
+            pair_put<DIM>(accp, p, r);
+          }
         }
       }
     }
@@ -1012,46 +1036,53 @@ __device__ __forceinline__ void group_advect(const MixK &m, const WinVar &v, con
 #pragma unroll
       for (int a = 0; a < DIM; ++a) st.c[a] = fma(h6, (double)accc[a], st.c[a]);
 #pragma unroll
-      for (int p = 0; p < DIM; ++p)
+      for (int p = 0; p < DIM; ++p) {
+        float2 d0[DIM], sum[DIM];
+        pair_get<DIM>(dpl, p, d0);
+        pair_get<DIM>(accp, p, sum);
 #pragma unroll
-        for (int a = 0; a < DIM; ++a) {
-          const int o = (p * DIM + a) * kBlock;
-          // k1 + 2k2 + 2k3 + k4, rounded as the in-loop fma(1, k4, sum) would
-          dpl[o] = fma2(h6f, fma2(one, kd[p][a], accp[o]), dpl[o]);
-        }
+        for (int a = 0; a < DIM; ++a)  // k1 + 2k2 + 2k3 + k4, rounded as the in-loop fma(1, k4, sum) would
+          d0[a] = fma2(h6f, fma2(one, kd[p][a], sum[a]), d0[a]);
+        pair_put<DIM>(dpl, p, d0);
+      }
     } else if constexpr (INTEG == FTLE_EULER) {
 #pragma unroll
       for (int a = 0; a < DIM; ++a) st.c[a] = fma(h, (double)kc[a], st.c[a]);
 #pragma unroll
-      for (int p = 0; p < DIM; ++p)
+      for (int p = 0; p < DIM; ++p) {
+        float2 d0[DIM];
+        pair_get<DIM>(dpl, p, d0);
 #pragma unroll
-        for (int a = 0; a < DIM; ++a) {
-          const int o = (p * DIM + a) * kBlock;
-          dpl[o] = fma2(bc2(hf), kd[p][a], dpl[o]);
-        }
+        for (int a = 0; a < DIM; ++a) d0[a] = fma2(bc2(hf), kd[p][a], d0[a]);
+        pair_put<DIM>(dpl, p, d0);
+      }
     } else {  // AB2, Euler on the first step (integrate.py:240-246)
       if (i == 0) {
 #pragma unroll
         for (int a = 0; a < DIM; ++a) st.c[a] = fma(h, (double)kc[a], st.c[a]);
 #pragma unroll
-        for (int p = 0; p < DIM; ++p)
+        for (int p = 0; p < DIM; ++p) {
+          float2 d0[DIM];
+          pair_get<DIM>(dpl, p, d0);
 #pragma unroll
-          for (int a = 0; a < DIM; ++a) {
-            const int o = (p * DIM + a) * kBlock;
-            dpl[o] = fma2(bc2(hf), kd[p][a], dpl[o]);
-          }
+          for (int a = 0; a < DIM; ++a) d0[a] = fma2(bc2(hf), kd[p][a], d0[a]);
+          pair_put<DIM>(dpl, p, d0);
+        }
       } else {
 #pragma unroll
         for (int a = 0; a < DIM; ++a)
           st.c[a] = fma(h, 1.5 * (double)kc[a] - 0.5 * (double)st.kcp[a], st.c[a]);
 #pragma unroll
-        for (int p = 0; p < DIM; ++p)
+        for (int p = 0; p < DIM; ++p) {
+          float2 d0[DIM];
+          pair_get<DIM>(dpl, p, d0);
 #pragma unroll
           for (int a = 0; a < DIM; ++a) {
-            const int o = (p * DIM + a) * kBlock;
             const float2 prev = make_float2(st.kdp[2 * p][a], st.kdp[2 * p + 1][a]);
-            dpl[o] = fma2(bc2(hf), fma2(bc2(1.5f), kd[p][a], mul2(bc2(-0.5f), prev)), dpl[o]);
+            d0[a] = fma2(bc2(hf), fma2(bc2(1.5f), kd[p][a], mul2(bc2(-0.5f), prev)), d0[a]);
           }
+          pair_put<DIM>(dpl, p, d0);
+        }
       }
 #pragma unroll
       for (int a = 0; a < DIM; ++a) st.kcp[a] = kc[a];
@@ -1082,13 +1113,15 @@ __device__ __forceinline__ void group_advect(const MixK &m, const WinVar &v, con
 #pragma unroll
   for (int a = 0; a < DIM; ++a) st.wraps[a] = wraps[a * kBlock];
 #pragma unroll
-  for (int p = 0; p < DIM; ++p)
+  for (int p = 0; p < DIM; ++p) {
+    float2 d0[DIM];
+    pair_get<DIM>(dpl, p, d0);
 #pragma unroll
     for (int a = 0; a < DIM; ++a) {
-      const float2 dv = dpl[(p * DIM + a) * kBlock];
-      st.d[2 * p][a] = dv.x;
-      st.d[2 * p + 1][a] = dv.y;
+      st.d[2 * p][a] = d0[a].x;
+      st.d[2 * p + 1][a] = d0[a].y;
     }
+  }
 }
 
 // Final positions x_k = c + wraps*period + d_k and the FP64 FTLE epilogue.
@@ -1319,7 +1352,8 @@ __global__ void sort_place_kernel(const int *__restrict__ keys, long long N, int
 // short (3D warps queue 2 to 17 of 192 neighbours a stage) saves instructions but was 4 to 8 %
 // slower wherever both versions of the pass were present.  So registers and code are what is
 // saved: period counts in shared memory, rare cases behind warp-wide branches.  128^3 groups x
-// 200 steps: 70.2 -> 66.9 ms; 2D, 131,072 groups x 80 steps: 826 -> 772 us.
+// 200 steps: 70.2 -> 64.9 ms (0.6 of it between chunks); 2D, 131,072 groups x 80 steps: 826 ->
+// 756 us.
 // Blocks of kBlock threads resident per SM that the register budget is sized for
 // (measured on B200): 4 in 3D; in 2D the persistent batched kernel runs 8 (the
 // turbulence windows keep most neighbours in their cell and gain from latency
@@ -1356,8 +1390,8 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks<DIM>)
   extern __shared__ __align__(16) unsigned char dyn_smem[];
   const BlockSmem<DIM> sm(dyn_smem);
   float *smem_slots = sm.slots;
-  float2 *acc = reinterpret_cast<float2 *>(sm.acc) + threadIdx.x;
-  float2 *dsm = reinterpret_cast<float2 *>(sm.d) + threadIdx.x;
+  float2 *acc = reinterpret_cast<float2 *>(sm.acc);
+  float2 *dsm = reinterpret_cast<float2 *>(sm.d);
   int *wraps = sm.wraps + threadIdx.x;
   const int lane = threadIdx.x & 31;
   WarpQueue<DIM> &wq = sm.queue[threadIdx.x >> 5];
@@ -1428,8 +1462,8 @@ __global__ void __launch_bounds__(kBlock, kMinBlocksPersistent<DIM>)
   const BlockSmem<DIM> sm(dyn_smem);
   __shared__ int s_item;
   float *smem_slots = sm.slots;
-  float2 *acc = reinterpret_cast<float2 *>(sm.acc) + threadIdx.x;
-  float2 *dsm = reinterpret_cast<float2 *>(sm.d) + threadIdx.x;
+  float2 *acc = reinterpret_cast<float2 *>(sm.acc);
+  float2 *dsm = reinterpret_cast<float2 *>(sm.d);
   int *wraps = sm.wraps + threadIdx.x;
   const int lane = threadIdx.x & 31;
   WarpQueue<DIM> &wq = sm.queue[threadIdx.x >> 5];
