@@ -774,7 +774,7 @@ __device__ __forceinline__ void eval_group(const MixK &m, const Header16 &hd,
       for (int i = 0; i < NC; ++i) Ac[i] = c == 0 ? Auv[i].x : (c == 1 ? Auv[i].y : Aw[i]);
       float2 dp = poly_diff_pair<DIM>(Ac, fc[0], g[c], F, dl);
       if constexpr (FX) dp = mul2(bc2(hd.scale[c]), dp);
-      kd[p][c] = DIM == 2 ? dp : make_float2(cin ? dp.x : 0.0f, cin ? dp.y : 0.0f);
+      kd[p][c] = dp;
     }
     const int k0 = 2 * p, k1 = 2 * p + 1;
     // 2D stores every neighbour's F without a branch (most warps have an off-cell
@@ -800,8 +800,8 @@ __device__ __forceinline__ void eval_group(const MixK &m, const Header16 &hd,
       }
     }
   }
-  // centroids outside the grid leave zeros; in 3D by selects above (a branch measured 1 % slower)
-  if (DIM == 2 && !__all_sync(0xffffffffu, cin)) {
+  // centroids outside the grid leave zeros
+  if (!__all_sync(0xffffffffu, cin)) {
 #pragma unroll
     for (int p = 0; p < DIM; ++p)
 #pragma unroll
@@ -1352,7 +1352,7 @@ __global__ void sort_place_kernel(const int *__restrict__ keys, long long N, int
 // short (3D warps queue 2 to 17 of 192 neighbours a stage) saves instructions but was 4 to 8 %
 // slower wherever both versions of the pass were present.  So registers and code are what is
 // saved: period counts in shared memory, rare cases behind warp-wide branches.  128^3 groups x
-// 200 steps: 70.2 -> 64.9 ms (0.6 of it between chunks); 2D, 131,072 groups x 80 steps: 826 ->
+// 200 steps: 70.2 -> 64.1 ms (0.6 of it between chunks); 2D, 131,072 groups x 80 steps: 826 ->
 // 756 us.
 // Blocks of kBlock threads resident per SM that the register budget is sized for
 // (measured on B200): 4 in 3D; in 2D the persistent batched kernel runs 8 (the
