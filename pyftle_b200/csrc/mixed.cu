@@ -25,6 +25,8 @@
 #include <cuda_fp16.h>
 #include <math.h>
 
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace ftle {
@@ -672,7 +674,10 @@ __device__ __forceinline__ void pair_put(float2 *base, int p, const float2 *v) {
 template <int DIM>
 struct WarpQueue {
   static constexpr int kCap = 32 * 2 * DIM;
-  int dst[kCap];
+  // 16 bits in 3D: with the counts of removed periods beside the queue, 4 blocks then fit the
+  // 132 KB carve-out and L1 keeps 124 KB, not 92 (128^3 groups x 200 steps 64.1 -> 63.1 ms).  In
+  // 2D the narrow accesses cost more than that gives (turbulence batch 2.6 % slower).
+  std::conditional_t<DIM == 3, unsigned short, int> dst[kCap];
   int ci[DIM][32];  // centroid cell of each lane's group
 };
 
@@ -956,8 +961,8 @@ __device__ __forceinline__ void group_from_positions(const MixK &m, const WinVar
 // Advect one group through steps [i0, i1) of the window.  The neighbour offsets
 // (dpl) and the RK4 accumulators (accp) live in this thread's shared-memory
 // columns by neighbour pair p = k/2 (pair_get: 16 bytes an access, 6 instead of 9 a
-// stage in 3D), the counts of removed periods (wraps) in int planes.
-template <int DIM, int MODE, int INTEG, int STORAGE>
+// stage in 3D), with WRAPS the counts of removed periods (wraps) in int planes.
+template <int DIM, int MODE, int INTEG, int STORAGE, bool WRAPS>
 __device__ __forceinline__ void group_advect(const MixK &m, const WinVar &v, const Header16 &hd,
                                              GroupState<DIM> &st, int i0, int i1,
                                              float *smem_slots, float2 *accp, float2 *dpl,
@@ -985,7 +990,8 @@ __device__ __forceinline__ void group_advect(const MixK &m, const WinVar &v, con
   }
 
 #pragma unroll
-  for (int a = 0; a < DIM; ++a) wraps[a * kBlock] = st.wraps[a];
+  for (int a = 0; a < DIM; ++a)
+    if constexpr (WRAPS) wraps[a * kBlock] = st.wraps[a];
   constexpr int NST = INTEG == FTLE_RK4 ? 4 : 1;
   using Times = StepTimes<MODE, INTEG>;
   Times times;
@@ -1102,16 +1108,17 @@ __device__ __forceinline__ void group_advect(const MixK &m, const WinVar &v, con
         const double lo = m.w.g.origin[a], hi = lo + m.period[a];
         if (st.c[a] < lo) {
           st.c[a] += m.period[a];
-          --wraps[a * kBlock];
+          --(WRAPS ? wraps[a * kBlock] : st.wraps[a]);
         } else if (st.c[a] >= hi) {
           st.c[a] -= m.period[a];
-          ++wraps[a * kBlock];
+          ++(WRAPS ? wraps[a * kBlock] : st.wraps[a]);
         }
       }
     }
   }
 #pragma unroll
-  for (int a = 0; a < DIM; ++a) st.wraps[a] = wraps[a * kBlock];
+  for (int a = 0; a < DIM; ++a)
+    if constexpr (WRAPS) st.wraps[a] = wraps[a * kBlock];
 #pragma unroll
   for (int p = 0; p < DIM; ++p) {
     float2 d0[DIM];
@@ -1352,7 +1359,7 @@ __global__ void sort_place_kernel(const int *__restrict__ keys, long long N, int
 // short (3D warps queue 2 to 17 of 192 neighbours a stage) saves instructions but was 4 to 8 %
 // slower wherever both versions of the pass were present.  So registers and code are what is
 // saved: period counts in shared memory, rare cases behind warp-wide branches.  128^3 groups x
-// 200 steps: 70.2 -> 64.1 ms (0.6 of it between chunks); 2D, 131,072 groups x 80 steps: 826 ->
+// 200 steps: 70.2 -> 63.1 ms (0.6 of it between chunks); 2D, 131,072 groups x 80 steps: 826 ->
 // 756 us.
 // Blocks of kBlock threads resident per SM that the register budget is sized for
 // (measured on B200): 4 in 3D; in 2D the persistent batched kernel runs 8 (the
@@ -1363,13 +1370,19 @@ template <int DIM>
 constexpr int kMinBlocks = 4;
 template <int DIM>
 constexpr int kMinBlocksPersistent = DIM == 2 ? 8 : 4;
+// Whether the counts of removed periods are in shared memory in the batched kernel: 8 blocks
+// in 2D would take the 164 KB carve-out with them, and take the 132 KB one without (24 windows
+// at rms speed 0.02 15.9 -> 15.75 ms, at 0.1 20.6 -> 19.6 ms, at 0.3 29.9 -> 28.5 ms).
+template <int DIM>
+constexpr bool kPersistentWraps = DIM == 3;
 
 template <int DIM>
 struct BlockSmem {
   static constexpr int kCol = 2 * DIM * DIM * kBlock;
-  static constexpr size_t kBytes = 3 * kCol * sizeof(float) +
-                                   (kBlock / 32) * sizeof(WarpQueue<DIM>) +
-                                   DIM * kBlock * sizeof(int);
+  static constexpr size_t kWraps = DIM * kBlock * sizeof(int);
+  static constexpr size_t kBytes =
+      3 * kCol * sizeof(float) + (kBlock / 32) * sizeof(WarpQueue<DIM>) + kWraps;
+  static constexpr size_t kPersistentBytes = kBytes - (kPersistentWraps<DIM> ? 0 : kWraps);
   float *slots, *acc, *d;
   int *wraps;
   WarpQueue<DIM> *queue;
@@ -1412,7 +1425,7 @@ __global__ void __launch_bounds__(kBlock, kMinBlocks<DIM>)
   } else {
     g = state_load<DIM>(buf, j, st, AB2);
   }
-  group_advect<DIM, MODE, INTEG, STORAGE>(m, v, hd, st, i0, i1, smem_slots, acc, dsm, wraps, wq,
+  group_advect<DIM, MODE, INTEG, STORAGE, true>(m, v, hd, st, i0, i1, smem_slots, acc, dsm, wraps, wq,
                                           lane);
   if (!active) return;
   if (last) {
@@ -1482,13 +1495,13 @@ __global__ void __launch_bounds__(kBlock, kMinBlocksPersistent<DIM>)
     const long long j = v.group_order ? v.group_order[slot] : slot;
     GroupState<DIM> st;
     group_from_positions<DIM>(m, v, j, st);
-    group_advect<DIM, MODE, INTEG, STORAGE>(m, v, hd, st, 0, v.num_steps, smem_slots, acc, dsm,
-                                            wraps, wq, lane);
+    group_advect<DIM, MODE, INTEG, STORAGE, kPersistentWraps<DIM>>(
+        m, v, hd, st, 0, v.num_steps, smem_slots, acc, dsm, wraps, wq, lane);
     if (active) group_finish<DIM>(m, v, j, st);
   }
 }
 
-// Allow the kernel's dynamic shared memory (33 KB for a 3D block, 16 KB in 2D, under
+// Allow the kernel's dynamic shared memory (31.5 KB for a 3D block, 15 KB in 2D, under
 // the 48 KB default today; set anyway so a larger layout needs no other change);
 // called once per kernel instance.
 template <typename Kernel>
@@ -1504,10 +1517,11 @@ static void launch_persistent(const MixK &m, int integ, const WinVar *wins,
 #define LP(I)                                                                              \
   do {                                                                                     \
     static const bool attr_set = set_smem_attr(windows_persistent_kernel<DIM, MODE, I, STORAGE>, \
-                                               BlockSmem<DIM>::kBytes);                    \
+                                               BlockSmem<DIM>::kPersistentBytes);          \
     (void)attr_set;                                                                        \
     windows_persistent_kernel<DIM, MODE, I, STORAGE>                                       \
-        <<<ctas, kBlock, BlockSmem<DIM>::kBytes, st>>>(m, wins, items, num_items, counter); \
+        <<<ctas, kBlock, BlockSmem<DIM>::kPersistentBytes, st>>>(m, wins, items, num_items,    \
+                                                               counter);                 \
   } while (0)
   if (integ == FTLE_EULER)
     LP(FTLE_EULER);
