@@ -221,9 +221,9 @@ class WindowBatch:
                    for w, d in zip(self.windows, self.desc))
 
     def _plan(self, order: int) -> torch.Tensor:
-        key = (order, self._copies)  # plans that a captured graph may read stay
+        key = (order, self._copies)
         if key in self._plans:
-            return self._plans[key]
+            return self._plans[key][0]
         lib = _lib.load()
         nbytes = lib.ftle_windows_plan_bytes(self.desc, self.count)
         if nbytes < 0:
@@ -236,7 +236,9 @@ class WindowBatch:
         _lib.call("ftle_windows_plan_ordered", self.desc, self.count, int(order), orders,
                   host.ctypes.data_as(ctypes.c_void_p), nbytes)
         dev = torch.from_numpy(host).to(self.windows[0].positions.device)
-        self._plans[key] = dev
+        # a captured graph and a run in flight read the plan and the buffers it points at:
+        # both stay, also when the windows are bound to others
+        self._plans[key] = (dev, self._bound)
         return dev
 
     def _view(self, t: torch.Tensor) -> torch.Tensor:
@@ -259,10 +261,15 @@ class WindowBatch:
 
     def run(self, schedule: Optional[Schedule] = None, stream=None) -> List[torch.Tensor]:
         sch = schedule or self.schedule
+        on_stream = lambda: (torch.cuda.stream(stream) if stream is not None  # noqa: E731
+                             else contextlib.nullcontext())
         if self.spatial_order and not self._copies and self._rebound():
-            self._bind(True)
+            # copies from the pool of the stream that fills them: memory recycled there is free
+            # once that stream reaches it, another stream's may still be in use
+            with on_stream():
+                self._bind(True)
         plan = self._plan(sch.order)
-        with torch.cuda.stream(stream) if stream is not None else contextlib.nullcontext():
+        with on_stream():
             if self._copies:
                 self._gather()
             _lib.call("ftle_windows_run_mixed", self.desc, self.count, plan.data_ptr(),
