@@ -39,15 +39,6 @@ from pyftle_b200 import _lib
 from pyftle_b200._device import as_device_f64, ptr, require_cuda, stream_ptr, to_host
 
 
-def _extent(x: np.ndarray):
-    """(min, max) of a coordinate array, in one threaded pass where torch can read it."""
-    if x.dtype == np.float64 and x.flags.writeable and x.flags.aligned and x.size \
-            and all(s > 0 for s in x.strides):
-        lo, hi = torch.aminmax(torch.from_numpy(x))
-        return np.float64(lo.item()), np.float64(hi.item())
-    return np.min(x), np.max(x)
-
-
 @dataclass(frozen=True)
 class GridSpec:
     """Regular grid: nodes per axis, origin and spacing (C-ABI ``ftle_grid``)."""
@@ -79,7 +70,9 @@ class GridSpec:
             raise ValueError(f"points must have shape ({dim}, nodes)")
         origin, spacing = [], []
         for a in range(dim):
-            ax = np.linspace(*_extent(pts[a]), grid_shape[a])
+            # numpy: torch's threads are gone in a forked process, where its reductions would wait
+            # for them forever
+            ax = np.linspace(np.min(pts[a]), np.max(pts[a]), grid_shape[a])
             origin.append(float(ax[0]))
             spacing.append(float((ax[-1] - ax[0]) / (ax.shape[0] - 1)))
         return cls(tuple(int(n) for n in grid_shape), tuple(origin), tuple(spacing), periodic)
