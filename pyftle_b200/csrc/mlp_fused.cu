@@ -532,13 +532,15 @@ using namespace ftle::mlp;
 
 namespace {
 
-// Ring slots that fit beside the activations (two CTAs per SM up to hid = 256), 0 if the shape
-// is not one of the kernel's.
+// Dynamic shared memory a block may take: two CTAs per SM up to hid = kTwoCtaHid.
+constexpr size_t field_room(bool two_ctas) { return two_ctas ? 112 * 1024 : 224 * 1024; }
+
+// Ring slots that fit beside the activations, 0 if the shape is not one of the kernel's.
 int field_stages(int dim, int hid, int depth, int freqs) {
   if ((dim != 2 && dim != 3) || hid < 64 || hid > 384 || hid % 64 || depth < 1 ||
       depth > kMaxDepth || freqs < 32 || freqs % 32 || freqs > 64)
     return 0;
-  const size_t room = hid <= kTwoCtaHid ? 112 * 1024 : 224 * 1024;
+  const size_t room = field_room(hid <= kTwoCtaHid);
   const size_t fixed = field_smem(hid, depth, 2 * freqs, dim, 0);
   if (fixed > room) return 0;
   const size_t fit = (room - fixed) / ((size_t)weight_rows(hid) * kChunkK * 2);
@@ -557,8 +559,10 @@ void launch_field(const FieldArgs &a, cudaStream_t st) {
   const long long tiles = (a.n + kTile - 1) / kTile;
   const long long cap = (long long)kNumSMs * (P == 2 ? 2 : 1);
   const size_t smem = field_smem(a.hid, a.depth, 2 * a.freqs, DIM, a.stages);
+  // the limit is the instance's, the same on every call: one of this shape's size would be
+  // lowered by another thread's smaller network before this launch
   cudaFuncSetAttribute(surrogate_field_kernel<DIM, P>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)smem);
+                       (int)field_room(P == 2));
   surrogate_field_kernel<DIM, P><<<(unsigned)(tiles < cap ? tiles : cap), 64 + 128 * P, smem, st>>>(a);
 }
 
