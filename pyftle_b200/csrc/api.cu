@@ -69,6 +69,12 @@ int grid_from_abi(const ftle_grid *g, GridK *out) {
     out->rcp_lo[a] = fma(-out->rcp_hi[a], s, 1.0) / s;
     out->man_hi[a] = 1.0 / out->man[a];
     out->man_lo[a] = fma(-out->man_hi[a], out->man[a], 1.0) / out->man[a];
+    if (isinf(s)) {  // every finite dividend gives a zero of the quotient's sign
+      out->man[a] = out->man_hi[a] = copysign(1.0, s);
+      out->man_lo[a] = 0.0;
+      out->man_exp[a] = 4000;
+      out->div_min = 0x80000000u;
+    }
   }
   return FTLE_OK;
 }
