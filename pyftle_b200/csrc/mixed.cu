@@ -240,6 +240,9 @@ struct Encoder<FTLE_FX16> {
   __device__ Encoder(const Header16 &h, int c) {
     S = (double)h.scale[c];
     off = (double)h.offset[c];
+    // a range whose offset is past FP32 (the decoded values are -infinity whatever the code):
+    // the last code, as the division of the infinite difference gives
+    if (off < -3.5e38 && S < 3.5e38) off = -1.0e4 * S;
     hi = 1.0 / S;
     lo = fma(-hi, S, 1.0) / S;
   }
