@@ -57,6 +57,18 @@ def fourier_frequencies(num: int = 32, *, length: float = 2.0 * math.pi,
     return out
 
 
+def _weight_grad_splits(n: int, tiles: int, sms: int) -> int:
+    """Pieces of a weight gradient's contraction over n rows, with `tiles` 128 x 128 tiles.
+
+    As few turns of all SMs as leave at most 1024 rows to a piece: the tensor core truncates
+    where it adds to its FP32 accumulator, so the error grows with a piece's length
+    (512 x 512, 65,536 rows: pieces of 1024 rows 9e-7 of the gradient, one turn of 7,296 rows
+    7e-6).
+    """
+    turn = max(1, sms // tiles)
+    return turn * -(-n // (1024 * turn))
+
+
 @dataclass
 class _Layer:
     fan_in: int
@@ -302,9 +314,8 @@ class FlowMapMLP:
         for l in range(last, -1, -1):
             L = self.layers[l]
             x = ws["feat"] if l == 0 else ws[f"H{l - 1}"]
-            # dW_l (out_pad x fan_in) += G^T X  (contraction over the batch, split so that the
-            # 128 x 128 tiles' pieces fill the SMs once)
-            splits = max(1, sms // (-(-L.out_pad // 128) * -(-L.fan_in // 128)))
+            # dW_l (out_pad x fan_in) += G^T X  (contraction over the batch)
+            splits = _weight_grad_splits(n, -(-L.out_pad // 128) * -(-L.fan_in // 128), sms)
             _lib.call("ftle_mlp_gemm", ptr(g), ldg, 1, ptr(x), L.fan_in, 1,
                       ptr(self.grad_weight(l)), L.fan_in, L.out_pad, L.fan_in, n, splits, 1,
                       ptr(self.err), s)
