@@ -420,8 +420,8 @@ __global__ void features_kernel(const double *__restrict__ pts, long long n,
 // gradient (column sums of the BF16 dY) and the loss are added atomically.
 // A thread writes P consecutive columns of a row (P = 8: one 16-byte store, where lddy and dY
 // allow it, else 1), so a warp writes whole lines; a thread per row stored its 64 columns one
-// by one (65,536 rows: 41.9 us; now 8.5 us).  One block per SM: the loss and the bias gradients are
-// FP32 sums over blocks, whose rounding grows with their number.
+// by one (65,536 rows: 41.9 us; now 8.5 us).  One block per SM and per 256 rows: the loss and the
+// bias gradients are FP32 sums over blocks, whose rounding grows with their number.
 constexpr int kMseThreads = 512;
 template <int P>
 __global__ void __launch_bounds__(kMseThreads)
@@ -829,7 +829,8 @@ int ftle_mlp_mse_grad(const float *y, int32_t ldy, const float *target, int32_t 
   __nv_bfloat16 *d = static_cast<__nv_bfloat16 *>(dy);
   const bool wide = lddy % 8 == 0 && reinterpret_cast<uintptr_t>(dy) % 16 == 0;
   const int64_t need = (n * (wide ? lddy / 8 : lddy) + kMseThreads - 1) / kMseThreads;
-  const unsigned blocks = (unsigned)(need < kNumSMs ? need : kNumSMs);
+  const int64_t most = (n + 255) / 256 < kNumSMs ? (n + 255) / 256 : kNumSMs;
+  const unsigned blocks = (unsigned)(need < most ? need : most);
   if (wide)
     mse_grad_kernel<8><<<blocks, kMseThreads, 0, st>>>(y, ldy, target, outs, n, 1.0f / (float)n, d,
                                                        lddy, dbias, loss);
