@@ -15,7 +15,7 @@
 //       EPI_F32        store (or, split-K, add) FP32 C
 //       EPI_BIAS_SILU  z = acc + b: store z (FP32) and h = silu(z) (BF16)
 //       EPI_DSILU      g = acc * silu'(z_in): store g (BF16), column sums of g
-//                      (the bias gradient) atomically into colsum
+//                      (the bias gradient) into colsum, one atomic per CTA
 //       EPI_BIAS_F32   store acc + b (FP32)
 //     Their inputs and outputs pass through 6 KB of shared memory per warp and TMA (z_in of
 //     the next tile is fetched while this one is computed; C is added by TMA reductions).
@@ -261,19 +261,6 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
     };
     if (dsilu && lane == 0 && (int)blockIdx.x < total) fetch(blockIdx.x);
     float cs0 = 0.0f, cs1 = 0.0f;  // column sums of columns 2p, 2p+1 (p = lane % 16)
-    int cs_n0 = -1;
-    auto flush = [&]() {
-      if (cs_n0 >= 0) {
-        cs0 += __shfl_xor_sync(0xffffffffu, cs0, 16);
-        cs1 += __shfl_xor_sync(0xffffffffu, cs1, 16);
-        const int n = cs_n0 + c0 + 2 * (lane & 15);
-        if (lane < 16 && n < N) {  // N is even: both columns are inside
-          atomicAdd(epi.colsum + n, cs0);
-          atomicAdd(epi.colsum + n + 1, cs1);
-        }
-      }
-      cs0 = cs1 = 0.0f;
-    };
     int j = 0;
     uint32_t zph = 0;
     for (int u = blockIdx.x; u < total; u += gridDim.x, ++j) {
@@ -332,10 +319,6 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         }
         if (epi.colsum) {
           // the bias gradient sums the values the next GEMM consumes; rows past M are zero
-          if (cs_n0 != n0) {
-            flush();
-            cs_n0 = n0;
-          }
           const int p = lane & 15, r0 = lane & 16;
 #pragma unroll
           for (int r = 0; r < 16; ++r) {
@@ -370,7 +353,27 @@ __global__ void __launch_bounds__(kGemmThreads, 1)
         }
       }
     }
-    if (epi.colsum) flush();
+    if (dsilu && epi.colsum) {
+      // every unit of this CTA has the same columns (gemm_launch): its four warps of 32 columns
+      // add their rows first, so that the sum over CTAs rounds once per CTA
+      float2 *own = reinterpret_cast<float2 *>(tf);
+      cs0 += __shfl_xor_sync(0xffffffffu, cs0, 16);
+      cs1 += __shfl_xor_sync(0xffffffffu, cs1, 16);
+      if (lane < 16) own[lane] = make_float2(cs0, cs1);
+      // all epilogue warps come here, after bounded waits only
+      asm volatile("bar.sync 1, %0;" ::"n"(32 * kEpiWarps) : "memory");
+      const int n = (int)(blockIdx.x % tiles_n) * NT + c0 + 2 * lane;
+      if ((ew & 3) == 0 && lane < 16 && n < N) {  // N is even: both columns are inside
+#pragma unroll
+        for (int w = 1; w < 4; ++w) {
+          const float2 t = reinterpret_cast<const float2 *>(tf + w * kEpiBytes)[lane];
+          cs0 += t.x;
+          cs1 += t.y;
+        }
+        atomicAdd(epi.colsum + n, cs0);
+        atomicAdd(epi.colsum + n + 1, cs1);
+      }
+    }
     if (lane == 0) bulk_wait();
   }
   fence_before_sync();
@@ -726,7 +729,10 @@ int gemm_launch(const void *A, int lda, int a_trans, const void *B, int ldb, int
   if (splits > 1) e.accumulate = 1;
   const int tiles_m = (M + kTileM - 1) / kTileM, tiles_n = (N + NT - 1) / NT;
   const int total = tiles_m * tiles_n * splits;
-  const int grid = total < kNumSMs ? total : kNumSMs;  // persistent: one CTA per SM
+  int grid = total < kNumSMs ? total : kNumSMs;  // persistent: one CTA per SM
+  // column sums: a CTA's units share their columns (consecutive units run along a row of tiles)
+  if (epi.colsum && total > kNumSMs)
+    grid = tiles_n <= kNumSMs ? kNumSMs / tiles_n * tiles_n : tiles_n;
   cudaStream_t st = as_stream(stream);
   CUtensorMap tmA, tmB, tmF, tmH;
   int rc = operand_map(&tmA, A, a_trans != 0, M, K, lda, kTileM);
