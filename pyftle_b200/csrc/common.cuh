@@ -89,9 +89,10 @@ __device__ __forceinline__ int wrap_index(int q, int n) {
 // on the negative side (x the smallest) the other two are -x/2 +- d, and d^2 is half the
 // squared norm of B + x/2 I - 3/2 x P with P = adj(B - x I) / tr adj the projector on x's
 // eigenvector, which stays accurate when the two coincide.  B is scaled by a power of two.
-// Relative error 0.7-1.3e-16 (root mean square) over random, stretched, nearly isotropic and
-// nearly degenerate C = F F^T, as cyclic Jacobi rotations have (0.6-1.4e-16), at about a
-// tenth of their operations.
+// Relative error 0.5-0.9e-16 (root mean square, 3e-16 at most) over random, stretched, graded,
+// nearly isotropic and nearly degenerate C = F F^T, where cyclic Jacobi rotations have 0.6-1.4e-16
+// (5e-16); 0.2e-16 where C is all but diagonal, which rotations leave exact.  About a tenth of
+// their operations.
 static __device__ __noinline__ double lmax3_sym(double a00, double a01, double a02, double a11,
                                                 double a12, double a22) {
   const double off = fabs(a01) + fabs(a02) + fabs(a12);
@@ -102,9 +103,11 @@ static __device__ __noinline__ double lmax3_sym(double a00, double a01, double a
     return mx;
   }
   const double tr = a00 + a11 + a22;
-  double q = tr * (1.0 / 3.0);
-  q = fma(fma(-3.0, q, tr), 1.0 / 3.0, q);
+  const double q = tr * (1.0 / 3.0);
   double b0 = a00 - q, b1 = a11 - q, b2 = a22 - q;
+  // what rounding left of B's trace: next to a multiple of I it is as large as B
+  const double t = (b0 + b1 + b2) * (1.0 / 3.0);
+  b0 -= t, b1 -= t, b2 -= t;
   int e = ((__double2hiint(fabs(b0) + fabs(b1) + fabs(b2) + off) >> 20) & 0x7ff) - 1023;
   e = e > 1022 ? 1022 : e;
   const double down = __hiloint2double((1023 - e) << 20, 0);
@@ -140,7 +143,7 @@ static __device__ __noinline__ double lmax3_sym(double a00, double a01, double a
     const double f2 = fma(s, fma(a01, a02, -(a12 * r0)), a12);
     m = sqrt(fma(0.5, fma(e0, e0, fma(e1, e1, e2 * e2)), fma(f0, f0, fma(f1, f1, f2 * f2)))) - h;
   }
-  return fma(m, __hiloint2double((1023 + e) << 20, 0), q);
+  return q + fma(m, __hiloint2double((1023 + e) << 20, 0), t);
 }
 
 }  // namespace ftle
