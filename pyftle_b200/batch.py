@@ -81,9 +81,7 @@ class JudgeReport:
 
 @dataclass(frozen=True)
 class Schedule:
-    # 4 fill the chip (in 2D a pair of blocks each).  2D windows that stretch their groups over
-    # many cells gain from fewer, which leave each more L1: 64 turbulence windows at rms speed
-    # 0.02 131 ms with 4, 155 ms with 2; at 0.3 450 ms with 4, 348 ms with 2 (autotune)
+    # the kernel fits 4 blocks of 128 threads per SM in 3D, 8 in 2D
     ctas_per_sm: int = 4
     order: int = 1  # 1: longest windows first, 2: by start of the time range, 0: as given
 
@@ -390,8 +388,9 @@ class WindowBatch:
         if use_cache and self.shape_key in cache:
             self.schedule = Schedule(**cache[self.shape_key]["schedule"])
             return self.schedule
-        # 4 blocks (2D: pairs of blocks) per SM fill the chip
-        cands = list(candidates) if candidates else [Schedule(c, o) for c in (1, 2, 3, 4)
+        # blocks per SM the kernel can keep resident: 4 in 3D, up to 8 in 2D
+        ctas = (1, 2, 3, 4) if self.series.grid.dim == 3 else (2, 4, 6, 8)
+        cands = list(candidates) if candidates else [Schedule(c, o) for c in ctas
                                                      for o in (1, 2, 0)]
         timings = []
         for sch in cands:

@@ -1876,11 +1876,6 @@ int ftle_windows_run_mixed(const ftle_window *windows, int32_t count, void *devi
   if (ni == 0) return FTLE_OK;
   MixK m;
   mixed_setup(&windows[0], m);
-  // a 2D block takes half a 3D block's registers and shared memory: 2D launches blocks in
-  // pairs, so that the 4 per SM that fill the chip in 3D fill it in 2D (24 windows: 4 blocks
-  // 20.0 ms, 8 16.7; blocks of 256 threads with two items each 18.5, they spill)
-  int ctas = ctas_per_sm;
-  if (windows[0].grid.dim == 2) ctas = ctas < 4 ? 2 * ctas : 8;
   unsigned char *p = static_cast<unsigned char *>(device_plan);
   int *counter = reinterpret_cast<int *>(p + plan_offset_counter(count, ni));
   cudaStream_t st = as_stream(stream);
@@ -1889,7 +1884,7 @@ int ftle_windows_run_mixed(const ftle_window *windows, int32_t count, void *devi
   launch_persistent_any(m, windows[0].grid.dim, windows[0].time_mode, windows[0].integrator,
                         windows[0].storage, reinterpret_cast<const WinVar *>(p + plan_offset_wins()),
                         reinterpret_cast<const BatchItem *>(p + plan_offset_items(count)), (int)ni,
-                        counter, ctas * kNumSMs, st);
+                        counter, ctas_per_sm * kNumSMs, st);
   return check_launch("windows_persistent_kernel");
 }
 
