@@ -133,11 +133,35 @@ def _writes_overlap(windows: Sequence[WindowSpecRun]) -> bool:
     return False
 
 
+def _blocks_per_sm(series: SnapshotSeries, windows: Sequence[WindowSpecRun]) -> int:
+    """Blocks per SM of a batch that is given no schedule.
+
+    4 fill an SM in 3D; in 2D 8 fit.  8 hide more latency, but share the L1 that gathers of
+    stretched groups need, and spread few work items (128 groups) unevenly over the SMs.  So 8
+    from 9 items per SM on, where the groups' mean displacement in cells, which bounds how far a
+    flow that its grid resolves can stretch them, leaves them compact.  Times with 4 and 8 in
+    2D turbulence:
+      items    474 (62 cells) 1.14, 1.79 ms;   633 (438) 3.4, 5.0;   1,177 (FP16) 2.7, 3.3;
+               1,507 (473) 6.2, 5.7;   2,239 (287) 21.3, 20.9;   7,676 (44) 8.2, 6.3
+      cells    49 20.0, 15.8 ms;   486 331, 292;   904 56.5, 56.2;   971 416, 416;
+               2,914 563, 753
+    """
+    if series.grid.dim == 3:
+        return 4
+    runs = [(w.positions.shape[0] // 4, w.num_steps, abs(w.h)) for w in windows]
+    if sum(-(-n // 128) for n, _, _ in runs) < 9 * 148:
+        return 4
+    work = max(1, sum(n * steps for n, steps, _ in runs))
+    time = sum(n * steps * steps * h for n, steps, h in runs) / work
+    cells = series.peak_speed() * time / min(abs(s) for s in series.grid.spacing)
+    return 8 if cells <= 500.0 else 4
+
+
 class WindowBatch:
     def __init__(self, series: SnapshotSeries, windows: Sequence[WindowSpecRun], *,
                  integrator: str = "rk4", time_mode: str = "blend",
                  snapshot_t0: float = 0.0, snapshot_dt: float = 1.0,
-                 schedule: Schedule = Schedule(), spatial_order: bool = True):
+                 schedule: Optional[Schedule] = None, spatial_order: bool = True):
         if series.storage == _lib.F64:
             raise ValueError("batched windows run on the mixed-precision path (fx15/fp16/bf16)")
         self.series = series
@@ -193,7 +217,7 @@ class WindowBatch:
         self._bind(self.spatial_order and _writes_overlap(self.windows))
         self.graph: Optional[torch.cuda.CUDAGraph] = None
         self._plans = {}
-        self.schedule = schedule
+        self.schedule = schedule or Schedule(_blocks_per_sm(series, self.windows))
 
     # ------------------------------------------------------------------
     def _bind(self, copies: bool) -> None:

@@ -76,6 +76,15 @@ class SnapshotSeries:
     def nbytes(self) -> int:
         return self.packed.numel()
 
+    def peak_speed(self) -> float:
+        """Largest magnitude of a velocity component of a 16-bit series (waits for the device)."""
+        if self.storage in (_lib.FX15, _lib.FX16):  # the range stands in the header
+            ends = self.packed[:64].view(torch.float32).view(4, 4)[2:, :self.grid.dim]
+        else:
+            half = torch.float16 if self.storage == _lib.F16 else torch.bfloat16
+            ends = torch.stack(torch.aminmax(self.packed[256:].view(half)))
+        return float(ends.abs().max())
+
 
 def window_descriptor(series: SnapshotSeries, positions: torch.Tensor, ftle: Optional[torch.Tensor],
                       *, integrator: str, time_mode: str, h: float, num_steps: int,

@@ -55,3 +55,23 @@ def test_few_work_items_run_on_4_blocks_per_sm(dim, tmp_path):
     batch = _batch(dim)
     batch.run()
     assert _grid(batch.run, tmp_path) == 148 * 4
+
+
+@pytest.mark.parametrize("precision", ["fx15", "fx16", "fp16", "bf16"])
+@pytest.mark.parametrize("peak,blocks", [(0.5, 8), (1e5, 4)])
+def test_many_work_items_run_on_8_blocks_where_groups_stay_compact(precision, peak, blocks,
+                                                                   tmp_path):
+    peak = min(peak, 6e4) if precision == "fp16" else peak
+    n, groups = 16, 9 * 148 * 128
+    grid = GridSpec((n, n), (0.0, 0.0), (2 * math.pi / n,) * 2, True)
+    rng = np.random.default_rng(8)
+    snaps = rng.uniform(-0.25, 0.25, (3, 2, n * n)) * peak
+    snaps[1, 1, 7] = -peak
+    series = SnapshotSeries(grid, snaps, precision=precision)
+    assert series.peak_speed() == pytest.approx(peak, rel=2.0 ** -8)
+    seeds = torch.as_tensor(flows.seeds_2d(rng.uniform(0, 6, (groups, 2)), 1e-3), device="cuda")
+    batch = WindowBatch(series, [WindowSpecRun(seeds, 0.0, 0.01, 4, keep_positions=True)],
+                        snapshot_dt=0.1)
+    assert batch.schedule == Schedule(blocks, 1)
+    batch.run()
+    assert _grid(batch.run, tmp_path) == 148 * blocks
