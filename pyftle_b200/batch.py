@@ -374,8 +374,9 @@ class WindowBatch:
         g = self.series.grid
         steps = sorted(w.num_steps for w in self.windows)
         groups = sum(w.positions.shape[0] for w in self.windows) // (2 * g.dim)
+        # "blocks": what ctas_per_sm counts; 2D entries without it may count pairs of blocks
         return (f"d{g.dim}-{self.series.precision}-{self.kw['integrator']}-w{self.count}"
-                f"-g{int(np.log2(max(groups, 1)))}-s{steps[len(steps) // 2]}")
+                f"-g{int(np.log2(max(groups, 1)))}-s{steps[len(steps) // 2]}-blocks")
 
     # ------------------------------------------------------------------
     def capture(self, prologue=None) -> torch.cuda.CUDAGraph:
