@@ -25,6 +25,12 @@ from pyftle_b200._device import as_device_f64, ptr, stream_ptr
 from pyftle_b200.particles import NeighboringParticles
 
 
+def _initial_deltas(particles: NeighboringParticles) -> torch.Tensor:
+    if getattr(type(particles), "initial_deltas", None) is NeighboringParticles.initial_deltas:
+        return particles._delta_planes()  # read only: no copy
+    return particles.initial_deltas()
+
+
 def _check_stack(J: torch.Tensor, d: int) -> torch.Tensor:
     J = as_device_f64(J)
     if J.ndim != 3 or J.shape[1:] != (d, d):
@@ -38,7 +44,7 @@ def _jacobian(particles: NeighboringParticles, d: int) -> torch.Tensor:
     n = len(particles)
     J = torch.empty((n, d, d), dtype=torch.float64, device=particles.positions.device)
     _lib.call("ftle_flow_map_jacobian", d, ptr(particles.positions),
-              ptr(particles.initial_deltas()), n, ptr(J), stream_ptr())
+              ptr(_initial_deltas(particles)), n, ptr(J), stream_ptr())
     return J
 
 
@@ -102,5 +108,5 @@ def compute_ftle_from_positions(particles: NeighboringParticles, map_period: flo
     if out is None:
         out = torch.empty(n, dtype=torch.float64, device=particles.positions.device)
     _lib.call("ftle_from_positions", particles.dim, ptr(particles.positions),
-              ptr(particles.initial_deltas()), n, float(map_period), ptr(out), stream_ptr())
+              ptr(_initial_deltas(particles)), n, float(map_period), ptr(out), stream_ptr())
     return out

@@ -68,8 +68,8 @@ class NeighboringParticles:
         self.num_neighbors = self.positions.shape[1] * 2
         assert self.positions.shape[0] % self.num_neighbors == 0, (
             f"positions.shape[0] must be a multiple of {self.num_neighbors}")
-        # one launch for the separations (planes of a (dim, N, dim) block, which
-        # initial_deltas() hands out) and the centroid
+        # one launch for the separations (planes of a (dim, N, dim) block, which the FTLE kernels
+        # read as it is) and the centroid
         dim, dev = self.dim, self.positions.device
         n = self.positions.shape[0] // self.num_neighbors
         block = torch.empty((dim + 1, n, dim), dtype=torch.float64, device=dev)
@@ -109,9 +109,18 @@ class NeighboringParticles:
 
     def initial_deltas(self) -> torch.Tensor:
         """(dim, N, dim) stack [right-left; top-bottom (; front-back)] at t0 (C-ABI layout)."""
+        return torch.stack(self._delta_parts()).contiguous()
+
+    def _delta_parts(self):
         parts = [self.initial_delta_right_left, self.initial_delta_top_bottom]
         if self.dim == 3:
             parts.append(self.initial_delta_front_back)
+        return parts
+
+    def _delta_planes(self) -> torch.Tensor:
+        """initial_deltas() for calls that only read it: the block that the separations are planes
+        of, unless they were replaced."""
+        parts = self._delta_parts()
         first = parts[0]
         size = first.numel()
         if all(p.is_contiguous() and p.shape == first.shape
