@@ -240,14 +240,14 @@ struct Encoder<FTLE_FX16> {
   __device__ Encoder(const Header16 &h, int c) {
     S = (double)h.scale[c];
     off = (double)h.offset[c];
-    // a range whose offset is past FP32 (the decoded values are -infinity whatever the code):
-    // the last code, as the division of the infinite difference gives
-    if (off < -3.5e38 && S < 3.5e38) off = -1.0e4 * S;
+    // a range whose offset alone is past FP32, a negative S here: the last code, as the division
+    // of the infinite difference gives (the decoded values are -infinity whatever the code)
+    if (h.offset[c] == -INFINITY && h.scale[c] < INFINITY) S = -1.0;
     hi = 1.0 / S;
     lo = fma(-hi, S, 1.0) / S;
   }
   __device__ __forceinline__ unsigned short operator()(double v) const {
-    if (!(S > 0.0)) return 0;
+    if (!(S > 0.0)) return S < 0.0 && v == v ? 65535 : 0;
     const double a = v - off;
     const double q0 = fma(a, hi, a * lo);
     const double f = fma(fma(-q0, S, a), hi, q0);
