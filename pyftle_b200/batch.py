@@ -16,11 +16,12 @@ compact patch of the domain and its gathers share cache lines.  The kernel reads
 writes the caller's buffers through the order; where windows share a buffer that one of
 them writes, or a window's buffers were exchanged, each run instead gathers the seeds
 into that order, and scatters FTLE and final positions back window by window.  Without
-the copies' launches (two a window) 40 windows of 300 groups take 0.53 ms instead of
-0.96 ms, and the 2D turbulence batch of 24 windows 16.2 ms instead of 16.6 ms.  Per-group results are the same bits in either
-order.  ``autotune()`` times the schedule candidates (CTAs per SM,
-ordering) on the batch itself and keeps the fastest; results are cached per
-batch shape in ``~/.cache/pyftle_b200/tuning.json``.
+the copies' launches (two a window) 40 windows of 300 groups take 0.40 ms instead of
+0.94 ms, and the 2D turbulence batch of 24 windows 15.8 ms instead of 16.3 ms.  Per-group
+results are the same bits in either order.  Without a schedule the batch chooses its blocks
+per SM by a rule (``_blocks_per_sm``); ``autotune()`` times the schedule candidates (CTAs per
+SM, ordering) on the batch itself and keeps the fastest; results are cached per batch shape in
+``~/.cache/pyftle_b200/tuning.json``.
 """
 
 from __future__ import annotations
@@ -143,8 +144,8 @@ def _blocks_per_sm(series: SnapshotSeries, windows: Sequence[WindowSpecRun]) -> 
     2D turbulence:
       items    474 (62 cells) 1.14, 1.79 ms;   633 (438) 3.4, 5.0;   1,177 (FP16) 2.7, 3.3;
                1,507 (473) 6.2, 5.7;   2,239 (287) 21.3, 20.9;   7,676 (44) 8.2, 6.3
-      cells    49 20.0, 15.8 ms;   486 331, 292;   904 56.5, 56.2;   971 416, 416;
-               2,914 563, 753
+      cells    49 20.0, 15.8 ms;   486 331, 292;   777 388, 368;   971 416, 416;
+               1,263 450, 485;   2,914 563, 753
     """
     if series.grid.dim == 3:
         return 4
@@ -153,8 +154,8 @@ def _blocks_per_sm(series: SnapshotSeries, windows: Sequence[WindowSpecRun]) -> 
         return 4
     work = max(1, sum(n * steps for n, steps, _ in runs))
     time = sum(n * steps * steps * h for n, steps, h in runs) / work
-    cells = series.peak_speed() * time / min(abs(s) for s in series.grid.spacing)
-    return 8 if cells <= 500.0 else 4
+    cell = min(abs(s) for s in series.grid.spacing)
+    return 8 if series.peak_speed() * time <= 1000.0 * cell else 4
 
 
 class WindowBatch:

@@ -33,7 +33,7 @@ def test_3d_and_few_items_take_4_without_a_read_back():
     assert _blocks_per_sm(_series(2, None), []) == 4
 
 
-@pytest.mark.parametrize("peak,blocks", [(0.0, 8), (1.0, 8), (250.0, 8), (251.0, 4), (math.inf, 4),
+@pytest.mark.parametrize("peak,blocks", [(0.0, 8), (1.0, 8), (500.0, 8), (501.0, 4), (math.inf, 4),
                                          (math.nan, 4)])
 def test_many_items_take_8_where_they_stay_compact(peak, blocks):
     # one unit of time at `peak` over cells of 0.5
