@@ -314,7 +314,7 @@ int ftle_mlp_apply_displacement(const double *points, const float *y, int32_t ld
 /* 3D forms: points n x 4 FP64 (x, y, z, t); freq num_freq rows of 8 FP32
  * (kx, ky, kz, kt, phase, 0, 0, 0); tangents d/dx, d/dy, d/dz (each may be NULL);
  * the FTLE from the three tangents (columns 0..2) with lambda_max of the 3x3
- * Cauchy-Green tensor by Jacobi rotations; end positions n x 3. */
+ * Cauchy-Green tensor in closed form; end positions n x 3. */
 int ftle_mlp_features3(const double *points, int64_t n, const float *freq, int32_t num_freq,
                        void *features, void *tangent_x, void *tangent_y, void *tangent_z,
                        void *stream);

@@ -578,7 +578,7 @@ __global__ void features3_kernel(const double *__restrict__ pts, long long n,
 }
 
 // 3D FTLE of x -> x + s * net(x): F[r][j] = delta_rj + s * dY_r/dx_j (tangent j's
-// column r), C = F^T F, lambda_max by Jacobi rotations, ftle = log(sqrt(lambda))/|T|.
+// column r), C = F^T F, lambda_max in closed form (lmax3_sym), ftle = log(sqrt(lambda))/|T|.
 __global__ void jacobian_ftle3_kernel(const float *__restrict__ jx, const float *__restrict__ jy,
                                       const float *__restrict__ jz, int ld, long long n,
                                       double scale, double inv_T, double *__restrict__ ftle) {

@@ -31,16 +31,9 @@ struct Cell64 {
   double f[DIM];
 };
 
-// (x - origin) / spacing per axis as IEEE division rounds it, by multiplication.  With
-// 1/s = hi + lo (hi = RN(1/s), both from the host) q0 = RN(a hi + RN(a lo)) is within half
-// an ulp plus 2^-53 ulp of a/s, r = a - q0 s is exact in an FMA, and the last FMA's
-// argument q0 + r hi differs from a/s by less than the distance of any quotient of two
-// 53-bit numbers from a rounding boundary, so it rounds as a/s does.  That needs s and a
-// away from the ends of the exponent range: the host's div_range / div_base say where, and
-// a zero, an infinity, a NaN or any other dividend outside takes the division itself (4
-// instructions instead of ~12 and a subroutine's registers; see window_f64_kernel).
-// The same division for any dividend and spacing: on mantissas in [1, 2) (man_* from the
-// host), scaled afterwards.  Zeros, infinities and NaN keep their class and sign.
+// v / spacing for any dividend and spacing, as IEEE division rounds it: the reciprocal form of
+// grid_coords on mantissas in [1, 2) (man_* from the host), scaled afterwards in two factors.
+// Zeros, infinities and NaN keep their class and sign.
 __device__ __forceinline__ double div_scaled(double v, const GridK &g, int a) {
   const double sign = g.spacing[a] < 0.0 ? -1.0 : 1.0;
   if (v == 0.0 || !(fabs(v) <= 1.7976931348623157e308)) return v * sign;
@@ -61,6 +54,15 @@ __device__ __forceinline__ double div_scaled(double v, const GridK &g, int a) {
          __hiloint2double((1023 + e - half) << 20, 0);
 }
 
+// (x - origin) / spacing per axis as IEEE division rounds it, by multiplication.  With
+// 1/s = hi + lo (hi = RN(1/s), both from the host) q0 = RN(a hi + RN(a lo)) is within half
+// an ulp plus 2^-53 ulp of a/s, r = a - q0 s is exact in an FMA, and the last FMA's
+// argument q0 + r hi differs from a/s by less than the distance of any quotient of two
+// 53-bit numbers from a rounding boundary, so it rounds as a/s does.  That needs s and a
+// away from the ends of the exponent range: below div_min (the host's; every dividend where a
+// spacing is extreme) a dividend, zeros among them, takes div_scaled.  Infinities, NaN and
+// dividends that overflow come out not finite, which locate64 rejects as it does the quotient.
+// (4 instructions instead of ~12 and a subroutine's registers; see window_f64_kernel.)
 template <int DIM>
 __device__ __forceinline__ void grid_coords(const GridK &g, const double *x, double *p) {
   unsigned least = 0x7fffffffu;
@@ -541,10 +543,13 @@ __global__ void __launch_bounds__(2 * DIM * kGroups<DIM, MODE>, kBlocksPerSM<DIM
 
 // FTLE of every stride-th group of a window, straight from the snapshots as the caller has
 // them: the sample that judges a 16-bit window.  One thread per particle, one warp (3D: three)
-// per block, so that a sample spreads over the SMs; it is one FP64 chain long whatever its size
+// per block, so that a sample spreads over the SMs.  While it fits them it is one FP64 chain long
 // (1,311 groups of a 512^2 window, 80 steps: 0.17 ms on 164 of the chip's 592 schedulers), which
-// is why the caller runs it beside the window itself.  Records of the whole series for a sample
-// of 1 % took 76 us to write and twice the series' memory.
+// is why the caller runs it beside the window itself.  Beyond that the planes' scattered 8-byte
+// gathers cost more than records would, in 3D above all.  Alone, ms, against writing the records
+// and a window over them (which take twice the series' memory):
+//   2D, 80 steps: 1,311 groups 0.17, 0.24;   20,972 0.33, 0.33;   167,773 2.1, 1.3
+//   3D, 200 steps: 1,250 groups 1.5, 1.6;   20,972 4.1, 2.7;   167,773 43.9, 14.1
 template <int DIM>
 constexpr int kSampleGroups = DIM == 2 ? 8 : 16;
 

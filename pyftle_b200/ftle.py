@@ -8,7 +8,7 @@ inputs are uploaded):
 * ``compute_cauchy_green_2x2`` (C = F^T F, ftle.py:9-69) and
   ``compute_cauchy_green_3x3`` (C = F F^T, ftle.py:72-96);
 * ``max_eigenvalue_2x2`` (closed form, ftle.py:122-163) and
-  ``max_eigenvalue_3x3`` (symmetric Jacobi; the reference calls
+  ``max_eigenvalue_3x3`` (closed form for the symmetric part; the reference calls
   ``np.linalg.eigvals``, ftle.py:99-119);
 * ``compute_ftle_2x2/3x3(J, T)`` = ``(1/T) log(sqrt(lambda_max))``
   (ftle.py:166-233);
