@@ -21,9 +21,9 @@
 //     the next tile is fetched while this one is computed; C is added by TMA reductions).
 // These layers have K = 64-384, so the kernel is bound by the bytes of its FP32
 // pre-activations and BF16 activations.  65536 x 256 x 256 on one B200, before (16-byte-wide
-// TMA boxes, a thread storing its own row, scalar atomics) and now: BIAS_SILU 94 -> 34.8 us,
+// TMA boxes, a thread storing its own row, scalar atomics) and now: BIAS_SILU 94 -> 33.6 us,
 // DSILU with column sums 98 -> 36.9 us (134 MB each, 20 us at the measured copy rate), split-K
-// weight gradient 76 -> 26.6 us (event times, cold L2).
+// weight gradient 76 -> 27.6 us (event times, cold L2).
 // Every mbarrier wait is bounded; on timeout the kernel records an error in the
 // caller's error word, waits (bounded) for its copies and MMAs in flight, skips
 // the epilogue, frees its TMEM and returns.
