@@ -36,6 +36,8 @@ def _grid(run, tmp_path):
     prof.export_chrome_trace(path)
     with open(path) as f:
         events = json.load(f)["traceEvents"]
+    if not any(e.get("cat") == "kernel" for e in events):
+        pytest.skip("the profiler records no kernels on this machine")
     grids = [e["args"]["grid"] for e in events if "windows_persistent_kernel" in e.get("name", "")
              and "grid" in e.get("args", {})]
     assert len(grids) == 1
