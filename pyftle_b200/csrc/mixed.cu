@@ -1365,9 +1365,9 @@ __global__ void sort_place_kernel(const int *__restrict__ keys, long long N, int
 // 200 steps: 70.2 -> 63.1 ms (0.6 of it between chunks); 2D, 131,072 groups x 80 steps: 826 ->
 // 756 us.
 // Blocks of kBlock threads resident per SM that the register budget is sized for
-// (measured on B200): 4 in 3D; in 2D the persistent batched kernel runs 8 (the
-// turbulence windows keep most neighbours in their cell and gain from latency
-// hiding), the single-window kernel 4 (long, strongly stretching windows gather
+// (measured on B200): 4 in 3D; in 2D the persistent batched kernel fits 8 (windows
+// that keep most neighbours in their cell gain from latency hiding; the caller's
+// schedule says how many run), the single-window kernel 4 (long, strongly stretching windows gather
 // per neighbour and need the L1 that a larger shared-memory carve-out takes).
 template <int DIM>
 constexpr int kMinBlocks = 4;
